@@ -477,7 +477,7 @@ int bass_radix_sort_u64(uint64_t* keys, double* amps, int64_t n, int key_bits, v
   if ((n > 0 && (!keys || !amps)) || n < 0 || key_bits < 1 || key_bits > 64) return BASS_ERR_ARG;
   CHECK_WS(ws, ws_bytes, v);
   if (n > v.max_n) return BASS_ERR_WORKSPACE;
-  return status_of(run_radix_sort(keys, amps, n, nullptr, key_bits, v, ctrl, (cudaStream_t)stream, 0));
+  return status_of(run_radix_sort(keys, amps, n, key_bits, v, ctrl, (cudaStream_t)stream, 0));
 }
 
 int bass_merge_sorted(uint64_t* keys, double* amps, int64_t n, int64_t* n_out, void* ws, size_t ws_bytes,

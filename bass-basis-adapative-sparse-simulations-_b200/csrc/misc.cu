@@ -1,6 +1,6 @@
 // misc.cu -- streaming kernels of libbass_b200: reductions, fingerprints,
-// diagonal gates, state set-up / import / export, the LSD radix sort and the
-// merge of sorted duplicates, gathers, and the basis-rotation decision.
+// diagonal gates, state set-up / import and the merge of sorted duplicates,
+// gathers, and the basis-rotation decision.
 #include <math.h>
 
 #include "internal.h"
@@ -361,179 +361,6 @@ __global__ void k_gather_desc(const bass_state* in, bass_state* out, long long n
   out->rscale[1] = in->rscale[1];
   out->nq = in->nq;
   for (int p = 0; p < 64; ++p) { out->pos[p] = in->pos[p]; out->qat[p] = in->qat[p]; }
-}
-
-// export: true keys and scaled amplitudes (sorted afterwards)
-// (output amplitudes of the state's type; amp_type is what the caller expects)
-__global__ void k_export(const bass_state* st, uint64_t* ok, double* oa, long long max_n, int amp_type,
-                         bass_ctrl* c) {
-  __shared__ int8_t qat[64];
-  if (threadIdx.x < 64) qat[threadIdx.x] = st->qat[threadIdx.x];
-  __syncthreads();
-  const long long n = st->nnz;
-  if (n > max_n) return;
-  if (st->amp_type != amp_type) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) set_error(c, BASS_ERR_ARG);
-    return;
-  }
-  const double r0 = st->rscale[0], r1 = st->rscale[1];
-  const int c64 = amp_type == BASS_AMP_C64;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    ok[i] = true_key(st->keys[i], qat, 64);
-    amp_put(oa, i, amp_get(st->amps, i, c64, r0, r1), c64);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// LSD radix sort, 8-bit digits, stable (sparse_state.py:150-172 sorts 16-bit
-// digits; any stable LSD order gives the same result)
-// ---------------------------------------------------------------------------
-constexpr int kSortTile = 2048;
-
-__global__ void __launch_bounds__(256) k_rs_hist(const uint64_t* keys, const long long* n_dev,
-                                                 long long n_host, int shift, WsView ws) {
-  __shared__ unsigned int h[256];
-  const long long n = n_dev ? *n_dev : n_host;
-  const long long ntiles = (n + kSortTile - 1) / kSortTile;
-  if (ntiles > ws.sort_tiles || n > ws.max_n) return;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const long long lo = tile * kSortTile;
-    const long long hi = lo + kSortTile < n ? lo + kSortTile : n;
-    for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x)
-      atomicAdd(&h[(unsigned)(keys[i] >> shift) & 255u], 1u);
-    __syncthreads();
-    ws.sort_hist[(long long)threadIdx.x * ws.sort_tiles + tile] = h[threadIdx.x];
-    __syncthreads();
-  }
-}
-
-// exclusive scan of the digit-major histogram (256 x ntiles), one CTA
-__global__ void __launch_bounds__(1024) k_rs_scan(const long long* n_dev, long long n_host, WsView ws) {
-  __shared__ unsigned long long sPart[1024];
-  const long long n = n_dev ? *n_dev : n_host;
-  const long long ntiles = (n + kSortTile - 1) / kSortTile;
-  if (ntiles > ws.sort_tiles || n > ws.max_n) return;
-  const long long total = 256 * ntiles;
-  const long long per = (total + blockDim.x - 1) / blockDim.x;
-  const long long lo = threadIdx.x * per;
-  const long long hi = lo + per < total ? lo + per : total;
-  auto at = [&](long long k) -> unsigned int& {
-    const long long d = k / ntiles, t = k % ntiles;
-    return ws.sort_hist[d * ws.sort_tiles + t];
-  };
-  unsigned long long s = 0;
-  for (long long k = lo; k < hi; ++k) s += at(k);
-  sPart[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long run = 0;
-    for (int i = 0; i < (int)blockDim.x; ++i) {
-      const unsigned long long v = sPart[i];
-      sPart[i] = run;
-      run += v;
-    }
-  }
-  __syncthreads();
-  unsigned long long run = sPart[threadIdx.x];
-  for (long long k = lo; k < hi; ++k) {
-    const unsigned int v = at(k);
-    at(k) = (unsigned int)run;
-    run += v;
-  }
-}
-
-// P: the amplitude payload moved with each key (16 B complex128, 8 B complex64)
-template <typename P>
-__global__ void __launch_bounds__(256) k_rs_scatter(const uint64_t* ik, const P* ia, uint64_t* ok,
-                                                    P* oa, const long long* n_dev, long long n_host,
-                                                    int shift, WsView ws) {
-  __shared__ unsigned int cntw[8][257];
-  __shared__ unsigned int run[256];
-  __shared__ unsigned int base[256];
-  const long long n = n_dev ? *n_dev : n_host;
-  const long long ntiles = (n + kSortTile - 1) / kSortTile;
-  if (ntiles > ws.sort_tiles || n > ws.max_n) return;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    base[threadIdx.x] = ws.sort_hist[(long long)threadIdx.x * ws.sort_tiles + tile];
-    run[threadIdx.x] = 0;
-    const long long lo = tile * kSortTile;
-    for (int r = 0; r < kSortTile / 256; ++r) {
-      for (int d = threadIdx.x; d < 8 * 257; d += 256) (&cntw[0][0])[d] = 0;
-      __syncthreads();
-      const long long i = lo + r * 256 + threadIdx.x;
-      const bool valid = i < n;
-      uint64_t key = 0;
-      P amp{};
-      unsigned dig = 256;
-      if (valid) {
-        key = ik[i];
-        amp = ia[i];
-        dig = (unsigned)(key >> shift) & 255u;
-      }
-      const unsigned peers = __match_any_sync(0xffffffffu, dig);
-      const unsigned rank = __popc(peers & ((1u << lane) - 1));
-      if (rank == 0) cntw[w][dig] = __popc(peers);
-      __syncthreads();
-      if (valid) {
-        unsigned off = base[dig] + run[dig] + rank;
-        for (int ww = 0; ww < w; ++ww) off += cntw[ww][dig];
-        ok[off] = key;
-        oa[off] = amp;
-      }
-      __syncthreads();
-      {
-        unsigned add = 0;
-        for (int ww = 0; ww < 8; ++ww) add += cntw[ww][threadIdx.x];
-        run[threadIdx.x] += add;
-      }
-      __syncthreads();
-    }
-  }
-}
-
-template <typename P>
-__global__ void k_copy_entries(const uint64_t* ik, const P* ia, uint64_t* ok, P* oa,
-                               const long long* n_dev, long long n_host) {
-  const long long n = n_dev ? *n_dev : n_host;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    ok[i] = ik[i];
-    oa[i] = ia[i];
-  }
-}
-
-template <typename P>
-static cudaError_t radix_sort_t(uint64_t* keys, P* amps, long long n_host, const long long* n_dev, int key_bits,
-                                const WsView& ws, cudaStream_t s) {
-  const int grid = device().grid_small;
-  uint64_t* ks = keys;
-  P* as = amps;
-  uint64_t* kd = ws.tmp_keys;
-  P* ad = reinterpret_cast<P*>(ws.tmp_amps);
-  int passes = 0;
-  for (int shift = 0; shift < key_bits; shift += 8) {
-    KLAUNCH(S_SORT, s, k_rs_hist<<<grid, 256, 0, s>>>(ks, n_dev, n_host, shift, ws));
-    KLAUNCH(S_SORT, s, k_rs_scan<<<1, 1024, 0, s>>>(n_dev, n_host, ws));
-    KLAUNCH(S_SORT, s, k_rs_scatter<P><<<grid, 256, 0, s>>>(ks, as, kd, ad, n_dev, n_host, shift, ws));
-    uint64_t* tk = ks; ks = kd; kd = tk;
-    P* ta = as; as = ad; ad = ta;
-    ++passes;
-  }
-  if (passes & 1) KLAUNCH(S_SORT, s, k_copy_entries<P><<<grid, 256, 0, s>>>(ks, as, keys, amps, n_dev, n_host));
-  return cudaGetLastError();
-}
-
-// amps: complex128 pairs, or complex64 pairs when c64
-cudaError_t run_radix_sort(uint64_t* keys, double* amps, long long n_host, const long long* n_dev, int key_bits,
-                           const WsView& ws, bass_ctrl* ctrl, cudaStream_t s, int c64) {
-  (void)ctrl;
-  if (c64)
-    return radix_sort_t(keys, reinterpret_cast<unsigned long long*>(amps), n_host, n_dev, key_bits, ws, s);
-  return radix_sort_t(keys, reinterpret_cast<ulonglong2*>(amps), n_host, n_dev, key_bits, ws, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -921,19 +748,12 @@ cudaError_t run_import(bass_state* st, const uint64_t* keys, const double* amps,
   e = cudaMemcpyAsync(st_amps, amps, n * (c64 ? 2 * sizeof(float) : 2 * sizeof(double)), cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return e;
   KLAUNCH(S_SMALL, s, k_state_adopt<<<1, 1, 0, s>>>(st, st_keys, st_amps, cap, nq, n, amp_type));
-  e = run_radix_sort(st_keys, st_amps, n, nullptr, nq > 0 ? nq : 1, ws, ctrl, s, c64);
+  e = run_radix_sort(st_keys, st_amps, n, nq > 0 ? nq : 1, ws, ctrl, s, c64);
   if (e != cudaSuccess) return e;
   if ((e = zero_small(ws, s)) != cudaSuccess) return e;
   KLAUNCH(S_MERGE_RUNS, s, k_merge_runs<<<device().grid_small, 256, 0, s>>>(st_keys, st_amps, nullptr, n, ws, ctrl, c64));
   KLAUNCH(S_MERGE_RUNS, s, k_merge_out<<<device().grid_small, 256, 0, s>>>(st_keys, st_amps, ws, nullptr, st, c64));
   return cudaGetLastError();
-}
-
-cudaError_t run_export(const bass_state* st, uint64_t* ok, double* oa, int key_bits, const WsView& ws,
-                       bass_ctrl* ctrl, cudaStream_t s, int amp_type) {
-  KLAUNCH(S_SORT, s, k_export<<<device().grid_small, 256, 0, s>>>(st, ok, oa, ws.max_n, amp_type, ctrl));
-  return run_radix_sort(ok, oa, 0, reinterpret_cast<const long long*>(&st->nnz), key_bits, ws, ctrl, s,
-                        amp_type == BASS_AMP_C64);
 }
 
 cudaError_t run_merge_sorted(uint64_t* keys, double* amps, long long n, long long* n_out,
