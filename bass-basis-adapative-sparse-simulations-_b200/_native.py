@@ -52,21 +52,17 @@ PROF_SLOTS = 48
 KINDS = ["gate1", "rot1", "gate2", "perm", "plain", "rdm"]
 PASSES = ["hist", "hist2", "gather", "write", "rdm"]
 SLOT_NAMES = [f"k_tile<{k},{p}>" for k in KINDS for p in PASSES] + [
-    "k_partition", "k_select_coop", "k_select2", "k_tie_coop", "k_finalize", "reductions", "k_fingerprint",
-    "k_phase2q", "k_phase1q", "k_rdm_final", "radix_sort", "merge_runs", "bookkeeping", "select:level1",
-    "select:level2", "select:count", "select:settle+final", "select:two_level"]
-# select:* slots hold nanoseconds of k_select_coop's phases (block 0's clock,
-# barrier waits included; the last block's for settle+final) in prof_in and the
-# number of timed launches in prof_out; two_level counts (in prof_in) the
-# selections whose threshold needed the level-2 histogram, out of all
-# truncating selections (prof_out)
-SELECT_PHASE_SLOTS = (43, 44, 45, 46)
-SELECT_SPEC_SLOT = 47
-# the write step of gates, rotations and truncations is k_compact, counted in the write slot
-SLOT_NAMES[0 * 5 + 3] = "k_compact<gate1>"
-SLOT_NAMES[1 * 5 + 3] = "k_compact<rot1>"
-SLOT_NAMES[2 * 5 + 3] = "k_compact<gate2>"
-SLOT_NAMES[4 * 5 + 3] = "k_compact<plain>"
+    "k_partition", "k_op_zero", "unused32", "unused33", "unused34", "reductions", "k_fingerprint",
+    "k_phase2q", "k_phase1q", "k_rdm_final", "radix_sort", "merge_runs", "bookkeeping", "unused43",
+    "unused44", "unused45", "unused46", "unused47"]
+# gates, rotation steps, truncations and reorders: the staged route's passes
+# (its tile boundaries and sample are in the partition's slot), and the chip
+# route's one launch
+for _k, _name in enumerate(KINDS[:5]):
+    SLOT_NAMES[5 * _k] = f"k_op_eval<{_name}>"
+    SLOT_NAMES[5 * _k + 1] = f"k_op_settle<{_name}>"
+    SLOT_NAMES[5 * _k + 2] = f"k_op<{_name}>"
+    SLOT_NAMES[5 * _k + 3] = f"k_op_write<{_name}>"
 # the RDM qubits at low physical bits: one pass of k_rdm_low (the RDM kind's evaluation slot)
 SLOT_NAMES[5 * 5 + 0] = "k_rdm_low"
 
@@ -213,6 +209,7 @@ class Engine:
         self.scratch_f64 = torch.zeros(8, dtype=torch.float64, device=self.device)
         self.scratch_u64 = torch.zeros(8, dtype=torch.int64, device=self.device)
         self.pr_tie_tol = float(pr_tie_tol)
+        self._ws_for = {}
         self.reset()
 
     # -- plumbing ---------------------------------------------------------------
@@ -227,6 +224,19 @@ class Engine:
     @property
     def ws_ptr(self):
         return ctypes.c_void_p(_ptr(self.ws))
+
+    def ws_for(self, entries, slots):
+        """The workspace size to pass for an op on at most ``entries`` entries
+        with ``slots`` possible children each: the library takes the route for
+        the size this bounds (it never reads the entry count back)."""
+        need = max(int(entries), 1) * slots
+        b = self._ws_for.get(need)
+        if b is None:
+            if len(self._ws_for) > 64:
+                self._ws_for.clear()
+            b = min(self.ws_bytes, int(self.L.bass_workspace_bytes((need + 3) // 4, need, self.nq)))
+            self._ws_for[need] = b
+        return b
 
     def reset(self):
         tp = ctypes.c_void_p(_ptr(self.trace)) if self.trace is not None else None
@@ -310,6 +320,7 @@ class DevState:
         self.keys = torch.zeros(self.cap, dtype=torch.int64, device=eng.device)
         ft = torch.float32 if self.amp_type == AMP_C64 else torch.float64
         self.amps = torch.zeros(2 * self.cap, dtype=ft, device=eng.device)
+        self.nmax = 1   # an upper bound of the entry count, known without asking the device
         self.init(init_key)
 
     @property
@@ -325,6 +336,7 @@ class DevState:
                                                ctypes.c_void_p(_ptr(self.amps)), self.cap, self.eng.nq,
                                                ctypes.c_uint64(int(key)), self.amp_type, self.eng.stream),
               "bass_state_init")
+        self.nmax = 1
 
     def read_desc(self):
         return np.frombuffer(self.desc.cpu().numpy().tobytes(), dtype=STATE_DTYPE)[0]
@@ -365,6 +377,7 @@ class DevState:
         n = len(x)
         if n > self.cap:
             raise BassError("state capacity exceeded")
+        self.nmax = n
         real = np.float32 if self.amp_type == AMP_C64 else np.float64
         kx = torch.from_numpy(x.view(np.int64).copy()).to(eng.device) if n else self.keys
         ka = torch.from_numpy(a.view(real).copy()).to(eng.device) if n else self.amps
@@ -388,6 +401,16 @@ def swap(a: DevState, b: DevState):
     a.keys, b.keys = b.keys, a.keys
     a.amps, b.amps = b.amps, a.amps
     a.cap, b.cap = b.cap, a.cap
+    a.nmax, b.nmax = b.nmax, a.nmax
+
+
+def out_max(entries, slots, tr, cap):
+    """An upper bound of an op's output count: every child, or what its
+    truncation leaves (it cuts to k_keep when there are more than k_cond)."""
+    n = entries * slots
+    if tr.k_cond >= 0:
+        n = min(n, max(tr.k_cond, tr.k_keep))
+    return min(n, cap)
 
 
 def trunc(k_cond, k_keep, gamma_mode=0, renorm=0, mark_active=0, trace=0):

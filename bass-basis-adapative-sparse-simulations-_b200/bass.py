@@ -110,9 +110,12 @@ class BASS:
                     continue
                 tried[j] = V
                 u = nat.host_c128(V.conj().T)
+                n = state._cur.nmax
                 nat.check(eng.L.bass_rotate_step(state._cur.ptr, state._tmp.ptr, nat._host(u), j, self.k,
-                                                 int(self.trace), eng.ctrl_ptr, eng.ws_ptr, eng.ws_bytes,
+                                                 int(self.trace), eng.ctrl_ptr, eng.ws_ptr, eng.ws_for(n, 2),
                                                  eng.stream), "bass_rotate_step")
+                # either of the two states may be the current one now
+                state._cur.nmax = state._tmp.nmax = max(n, min(2 * n, self.k, state._cur.cap))
             state._touch()
             improved = False
             if tried:

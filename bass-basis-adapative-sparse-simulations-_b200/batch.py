@@ -218,6 +218,8 @@ class StatePool:
             st = self.states[c]
             by = {nat._ptr(d.desc): d for d in (st._cur, st._tmp, st._tmp2)}
             st._cur, st._tmp, st._tmp2 = by[int(self.pcur[c])], by[int(self.ptmp[c])], by[int(self.ptmp2[c])]
+            for d in by.values():
+                d.nmax = d.cap   # the segmented ops do not track their counts
             st._touch()
 
     def _kron(self, c, q1, q2):

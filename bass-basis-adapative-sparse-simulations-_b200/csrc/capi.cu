@@ -91,8 +91,8 @@ static Layout layout_for(long long max_n) {
   L.sort_tiles = max_n / 2048 + 2;
   size_t o = 0;
   L.counters = o; o += align256(64 * 8);
-  L.hist1 = o; o += align256((kHistBins + kHistGroups) * 4);
-  L.hist2 = o; o += align256((kHistBins + kHistGroups) * 4);
+  L.hist1 = o; o += align256(kHistBins * 4);
+  L.hist2 = o; o += align256(kHistBins * 4);
   L.sel = o; o += align256(sizeof(SelState));
   L.status = o; o += align256((size_t)L.max_tiles * 8);
   L.fp = o; o += align256(8 * 8);
@@ -100,12 +100,14 @@ static Layout layout_for(long long max_n) {
   L.part = o; o += align256((size_t)kMaxSets * (L.max_tiles + 1) * 6 * 8);
   const long long np = (long long)kMaxSets * L.max_tiles > 1024 ? (long long)kMaxSets * L.max_tiles : 1024;
   L.partials = o; o += align256((size_t)np * sizeof(Partial));
-  L.cand_bits = o; o += align256((size_t)max_n * 8);
-  L.cand_key = o; o += align256((size_t)max_n * 8);
+  // staged children: whole tiles of kTile positions (kStep of them counted in max_n)
+  const size_t stage = (size_t)max_n + (size_t)max_n / 128 + 4 * kTile;
+  L.cand_bits = o; o += align256(stage * 8);
+  L.cand_key = o; o += align256(stage * 8);
   L.tmp_keys = o; o += align256((size_t)max_n * 8);
-  L.tmp_amps = o; o += align256((size_t)max_n * 16);
-  L.stage_keys = o; o += align256((size_t)max_n * 8);
-  L.kmask = o; o += align256((size_t)max_n / 8 + 64);
+  L.tmp_amps = o; o += align256(stage * 16);
+  L.stage_keys = o; o += align256(stage * 8);
+  L.kmask = o; o += align256(stage / 8 + 64);
   L.sort_hist = o; o += align256((size_t)256 * L.sort_tiles * 4);
   L.total = o;
   return L;
@@ -557,7 +559,6 @@ static bool seg_common(const bass_seg_op& o, OpArgs* a) {
   a->out = o.out;
   a->ctrl = o.ctrl;
   a->nsets = 1;
-  a->fin = 1;
   a->k_cond = o.tr.k_cond;
   a->k_keep = o.tr.k_keep;
   a->tr = o.tr;
@@ -610,7 +611,7 @@ int bass_gate_1q_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t bat
   }
   if (!same_type(A)) return BASS_ERR_ARG;
   cudaError_t e = upload(bv.ops_a, A, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE1, bv.ops_a, n, A[0].c64, 0, 0, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE1, bv.ops_a, n, A[0].c64, bv.plan, s);
   return status_of(e);
 }
 
@@ -626,8 +627,6 @@ int bass_gate_2q_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t bat
     // pass 1: q2 to the lowest physical bit (a reorder, into tmp)
     A[i].out = o.tmp;
     A[i].q = o.q2;
-    A[i].write_mode = 2;
-    A[i].counter = 3;
     A[i].k_cond = -1;
     A[i].tr = bass_trunc{};
     A[i].tr.k_cond = -1;
@@ -640,8 +639,8 @@ int bass_gate_2q_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t bat
   if (!same_type(A)) return BASS_ERR_ARG;
   cudaError_t e = upload(bv.ops_a, A, s);
   if (e == cudaSuccess) e = upload(bv.ops_b, B, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_PERM, bv.ops_a, n, A[0].c64, 0, 0, bv.plan, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE2, bv.ops_b, n, A[0].c64, 0, 0, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_PERM, bv.ops_a, n, A[0].c64, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE2, bv.ops_b, n, A[0].c64, bv.plan, s);
   return status_of(e);
 }
 
@@ -670,7 +669,7 @@ int bass_topk_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t batch_
   }
   if (!same_type(A)) return BASS_ERR_ARG;
   cudaError_t e = upload(bv.ops_a, A, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_IDENT, bv.ops_a, n, A[0].c64, 0, 0, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_IDENT, bv.ops_a, n, A[0].c64, bv.plan, s);
   return status_of(e);
 }
 
@@ -691,7 +690,7 @@ int bass_rotate_step_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t
   }
   if (!same_type(A)) return BASS_ERR_ARG;
   cudaError_t e = upload(bv.ops_a, A, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_ROT1, bv.ops_a, n, A[0].c64, 1, 0, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_ROT1, bv.ops_a, n, A[0].c64, bv.plan, s);
   return status_of(e);
 }
 
@@ -703,7 +702,6 @@ int bass_rdm_1q_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t batc
     if (!seg_common(o, &A[i]) || !o.rho || o.num_qubits < 1 || o.num_qubits > BASS_MAX_QUBITS) return BASS_ERR_ARG;
     A[i].nsets = o.num_qubits;
     A[i].rho = o.rho;
-    A[i].fin = 0;
     if (o.num_qubits > max_nq) max_nq = o.num_qubits;
   }
   if (!same_type(A)) return BASS_ERR_ARG;

@@ -28,10 +28,6 @@ constexpr int kPerThread = kTile / kThreads;
 constexpr int kStep = kTile - 8;
 constexpr int kTilePad = kTile + 8;
 constexpr int kHistBins = 8192;      // 13-bit radix-select digits
-constexpr int kGroupBins = 128;      // bins per coarse group of a selection histogram
-constexpr int kHistGroups = kHistBins / kGroupBins;  // coarse counts stored after the bins
-constexpr int kCandSmem = 4096;      // candidates sorted in shared memory
-constexpr int kRankMax = 1024;       // candidates ranked by direct counting (one per thread of a selection block)
 constexpr int kMaxSets = 64;         // partition sets (one per qubit for RDMs)
 // RDM moments of the qubits at physical bits 0 .. kRdmLowBits - 1 come from
 // one pass over plain tiles plus a halo of kRdmHalo entries (k_rdm_low)
@@ -348,16 +344,21 @@ __device__ __forceinline__ uint64_t true_key(uint64_t y, const int8_t* qat, int 
   return x;
 }
 
-// Move physical bit t down to bit position gb (bits gb..t-1 shift up by one).
-// For gb = 0 this is "target to the lowest bit"; for gb = 1 bit 0 stays.
-__device__ __forceinline__ uint64_t zmove(uint64_t y, int t, int gb) {
-  uint64_t lomask = (1ULL << gb) - 1;
-  uint64_t bt = (y >> t) & 1ULL;
-  uint64_t hi = (t >= 63) ? 0 : (y >> (t + 1)) << (t + 1);
-  uint64_t midm = ((1ULL << t) - 1) & ~lomask;  // bits gb..t-1
-  uint64_t mid = y & midm;
-  return hi | (mid << 1) | (bt << gb) | (y & lomask);
-}
+// Moves physical bit t down to bit position GB (bits GB..t-1 shift up by one).
+// For GB = 0 this is "target to the lowest bit"; for GB = 1 bit 0 stays (t >= 1).
+template <int GB>
+struct ZMove {
+  uint64_t hi, mid;  // bits above t, bits GB..t-1
+  int t;
+  static constexpr uint64_t kLow = (1ULL << GB) - 1;
+  __device__ __forceinline__ explicit ZMove(int t_) : t(t_) {
+    hi = t >= 63 ? 0ULL : ~0ULL << (t + 1);
+    mid = ((1ULL << t) - 1) & ~kLow;
+  }
+  __device__ __forceinline__ uint64_t operator()(uint64_t y) const {
+    return (y & hi) | ((y & mid) << 1) | (((y >> t) & 1ULL) << GB) | (y & kLow);
+  }
+};
 
 // ---------------------------------------------------------------------------
 // warp-cooperative searches (32 probes per step)
@@ -588,40 +589,35 @@ struct Partial {
   long long pad[2];
 };
 
+// What later launches read of an op.
 struct SelState {
   long long n_out;       // children produced by the op (after drop rules)
   long long k_keep;
-  long long n_cand;      // children of the level-2 boundary bin (slot indices in ws.cand_bits)
-  unsigned long long t_bits;
-  unsigned long long t_key;  // ~0: every child at t_bits kept; else the largest kept true key there
   int do_trunc;
-  int stage;             // 0 keep all, 3 threshold resolved
-  int pad;               // K_IDENT guard: a zero amplitude was produced
+  int pad;               // K_IDENT guard: a zero amplitude was produced; 3: a renormalisation is pending
   double total;          // exact sum of |a|^2 over the op's output (truncating ops only)
   long long n_written;
   double kept;           // exact sum of |a|^2 over the kept children
-  double kept_p2;        // ... of |a|^4 (rotation steps)
-  int skip_write;        // the write pass has nothing to do (rejected rotation)
   int accept;            // rotation step: the candidate lowers PR
+  int unused;
   double pr_new;         // rotation step: PR of the candidate
-  int8_t qat[64];        // output qubit order, for the key tie-break at t_bits
 };
 
 struct WsView {
   long long* part;               // kMaxSets x (max_tiles + 1) x 6
   unsigned long long* status;    // max_tiles
-  unsigned int* hist1;           // kHistBins bins, then kHistGroups coarse counts
-  unsigned int* hist2;           // kHistBins bins, then kHistGroups coarse counts
+  unsigned int* hist1;           // kHistBins bins
+  unsigned int* hist2;           // kHistBins bins
   Partial* partials;             // kMaxSets x max_tiles
-  unsigned long long* cand_bits; // max_n: slot indices (boundary-bin candidates of a selection)
-  unsigned long long* cand_key;  // max_n
+  // the staged route's children, per region of a tile (op.cu), and scratch of others
+  unsigned long long* cand_bits; // |a|^2 patterns of the undecided children
+  unsigned long long* cand_key;  // their places (16 bits each); the sort's index buffers
   SelState* sel;
-  unsigned int* counters;        // 64 tile counters
-  uint64_t* tmp_keys;            // max_n; gate ops: the slot array (|a|^2 bits per child)
-  double2* tmp_amps;             // max_n; gate ops: the staged children's amplitudes
-  uint64_t* stage_keys;          // max_n; gate ops: the staged children's keys
-  uint8_t* kmask;                // max_n / 8 + 64: one bit per slot, kept by the selection (bit
-                                 // i & 7 of byte i >> 3; the count pass, then the boundary settle)
+  unsigned int* counters;        // 64 eight-byte counters
+  uint64_t* tmp_keys;            // max_n; the sort's and the merge's second key buffer
+  double2* tmp_amps;             // staged amplitudes; max_n: second amplitude buffer
+  uint64_t* stage_keys;          // staged keys
+  uint8_t* kmask;                // kept bits of the staged children, NS 8 words per region
   unsigned int* sort_hist;       // radix-sort tile histograms (256 x max_tiles)
   i128* red;                     // 1024 per-CTA reduction partials
   unsigned long long* fp;        // 8 fingerprint accumulators

@@ -12,6 +12,9 @@
 namespace bass {
 
 enum Kind { K_GATE1 = 0, K_ROT1 = 1, K_GATE2 = 2, K_PERM = 3, K_IDENT = 4, K_RDM = 5 };
+// Profile slots of a kind (kind * 5 + pass): P_HIST the staged evaluation,
+// P_HIST2 its settling, P_GATHER the chip route's one launch, P_WRITE the write
+// (and the compaction after a diagonal 1-qubit gate), P_RDM moments.
 enum Pass { P_HIST = 0, P_HIST2 = 1, P_GATHER = 2, P_WRITE = 3, P_RDM = 4 };
 
 // Op description passed by value to every tile kernel.
@@ -28,13 +31,11 @@ struct OpArgs {
   int drop_zero;  // K_IDENT: drop entries whose amplitude is exactly zero
   int guard;      // K_IDENT: run only if ws.sel->pad (zero flag) is set
   int prof;       // count entries into ctrl->prof_in / prof_out
-  int write_mode; // P_WRITE: 0 look-back + drop rule, 2 one child per entry
-  int fin;        // P_WRITE: the last CTA to finish writes the output descriptor (finalize_op)
-  int fin_mode;   // finalize_op: 0 gate / truncation, 1 rotation step
-  int commit;     // rotation step: the last CTA of the write pass also commits (swaps in an accepted candidate)
+  int fin_mode;   // 0 gate / truncation, 1 rotation step
+  int commit;     // rotation step: the op also commits (swaps in an accepted candidate)
   int j;          // rotation step: the rotated qubit
   long long k_cond, k_keep;
-  bass_trunc tr;  // finalize_op: gamma / renormalisation rules
+  bass_trunc tr;  // gamma / renormalisation rules
   int c64;        // the input state stores complex64 amplitudes (selects the kernels)
   int rdm_low;    // K_RDM: the qubits at physical bits below kRdmLowBits are left to k_rdm_low
   double* rho;    // RDM moments of a segmented RDM (4 per qubit)
@@ -51,9 +52,9 @@ struct SegPlan {
 };
 
 enum Slot {
-  S_PARTITION = 30, S_SELECT1 = 31, S_SELECT2 = 32, S_SELECT_EXACT = 33, S_FINALIZE = 34, S_REDUCE = 35,
+  S_PARTITION = 30, S_ZERO = 31, S_REDUCE = 35,
   S_FINGERPRINT = 36, S_PHASE2Q = 37, S_PHASE1Q = 38, S_RDM_FINAL = 39, S_SORT = 40, S_MERGE_RUNS = 41,
-  S_SMALL = 42, S_SLOT_HIST1 = 43, S_SLOT_HIST2 = 44, S_SLOT_GATHER = 45, S_SLOT_KEPT = 46
+  S_SMALL = 42
 };
 
 // Brackets one kernel launch: counts it and, when profiling is on, records
@@ -152,8 +153,8 @@ cudaError_t run_commit(bass_state* cur, bass_state* tmp, bass_ctrl* ctrl, const 
 
 // merge.cu, segmented: ops_dev holds nseg OpArgs (all of one amplitude type),
 // plan_dev is scratch for the block groups
-cudaError_t run_merge_op_seg(int kind, const OpArgs* ops_dev, int nseg, int c64, int fin_mode, int trace,
-                             SegPlan* plan_dev, cudaStream_t s);
+cudaError_t run_merge_op_seg(int kind, const OpArgs* ops_dev, int nseg, int c64, SegPlan* plan_dev, cudaStream_t s);
+cudaError_t run_seg_plan(const OpArgs* ops_dev, int nseg, int kind, SegPlan* plan_dev, cudaStream_t s);
 cudaError_t run_rdm_seg(const OpArgs* ops_dev, int nseg, int max_nq, int c64, SegPlan* plan_dev, cudaStream_t s);
 // the most segments one segmented launch takes on the current device
 cudaError_t seg_max_segments(int* out);
@@ -194,7 +195,5 @@ cudaError_t run_gather(const bass_state* in, bass_state* out, const int64_t* idx
 cudaError_t run_ctrl_init(bass_ctrl* c, uint64_t* trace, long long cap, double tol, cudaStream_t s);
 
 constexpr double kSigPmin = 1e-24;  // |a|^2 threshold of the significant-key fingerprint
-
-constexpr int kSmallWords = 64 /*counters*/ + 2 * kHistBins;  // zeroed at the start of every op
 
 }  // namespace bass

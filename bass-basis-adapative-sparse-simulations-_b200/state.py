@@ -39,6 +39,7 @@ class SparseState:
         self._cur = nat.DevState(self._eng, cap, key, at)
         self._tmp = nat.DevState(self._eng, cap, 0, at)
         self._tmp2 = nat.DevState(self._eng, cap, 0, at)
+        self._tmp.nmax = self._tmp2.nmax = cap   # scratch: whatever an op leaves there
         self._version = 0
         self._export = None
         self._order = None   # the reference's entry order (true keys) when not ascending
@@ -172,19 +173,24 @@ class SparseState:
             d = nat.host_c128([G[0, 0], G[1, 1]])
             nat.check(eng.L.bass_phase_1q(self._cur.ptr, self._tmp.ptr, nat._host(d), int(q), eng.ctrl_ptr,
                                           eng.ws_ptr, eng.ws_bytes, eng.stream), "bass_phase_1q")
+            self._tmp.nmax = self._cur.nmax   # the two may have changed places on the device
         else:
             g = nat.host_c128(G)
+            n = self._cur.nmax
             nat.check(eng.L.bass_gate_1q(self._cur.ptr, self._tmp.ptr, nat._host(g), int(q), tr, eng.ctrl_ptr,
-                                         eng.ws_ptr, eng.ws_bytes, eng.stream), "bass_gate_1q")
+                                         eng.ws_ptr, eng.ws_for(n, 2), eng.stream), "bass_gate_1q")
+            self._tmp.nmax = nat.out_max(n, 2, tr, self._tmp.cap)
             nat.swap(self._cur, self._tmp)
         self._rekeyed()
 
     def _apply_2q(self, G, q1, q2, tr):
         eng = self._eng
         g = nat.host_c128(G)
+        n = self._cur.nmax
         nat.check(eng.L.bass_gate_2q(self._cur.ptr, self._tmp.ptr, self._tmp2.ptr, nat._host(g), int(q1),
-                                     int(q2), tr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_bytes, eng.stream),
+                                     int(q2), tr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_for(n, 4), eng.stream),
                   "bass_gate_2q")
+        self._tmp.nmax, self._tmp2.nmax = n, nat.out_max(n, 4, tr, self._tmp2.cap)
         nat.swap(self._cur, self._tmp2)
         self._rekeyed()
 
@@ -193,9 +199,11 @@ class SparseState:
         truncation tr fused; the previous state is left in _tmp2."""
         eng = self._eng
         u = nat.host_c128(U4)
+        n = self._cur.nmax
         nat.check(eng.L.bass_rotate_2q(self._cur.ptr, self._tmp.ptr, self._tmp2.ptr, nat._host(u), int(q1),
-                                       int(q2), tr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_bytes, eng.stream),
+                                       int(q2), tr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_for(n, 4), eng.stream),
                   "bass_rotate_2q")
+        self._tmp.nmax, self._tmp2.nmax = n, nat.out_max(n, 4, tr, self._tmp2.cap)
         nat.swap(self._cur, self._tmp2)
         self._rekeyed()
 
@@ -230,8 +238,10 @@ class SparseState:
 
     def _topk(self, tr):
         eng = self._eng
-        nat.check(eng.L.bass_topk(self._cur.ptr, self._tmp.ptr, tr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_bytes,
+        n = self._cur.nmax
+        nat.check(eng.L.bass_topk(self._cur.ptr, self._tmp.ptr, tr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_for(n, 1),
                                   eng.stream), "bass_topk")
+        self._tmp.nmax = nat.out_max(n, 1, tr, self._tmp.cap)
         nat.swap(self._cur, self._tmp)
         self._rekeyed()
 
@@ -261,6 +271,7 @@ class SparseState:
         nat.check(eng.L.bass_gather(self._cur.ptr, self._tmp.ptr, nat.ctypes.c_void_p(nat._ptr(t)), len(idx),
                                     eng.ctrl_ptr, eng.stream), "bass_gather")
         torch.cuda.current_stream(eng.device).synchronize()
+        self._tmp.nmax = len(idx)
         nat.swap(self._cur, self._tmp)
         self._rekeyed()
 

@@ -320,7 +320,6 @@ def profile_step(a, circ, L, nat, BASS, torch, step_ms):
         kernels.append({"kernel": nat.SLOT_NAMES[s], "ms": round(float(ms[s]), 3), "launches": int(cnt[s]),
                         "share": round(float(ms[s] / ms.sum()), 4),
                         "gbs": round(nbytes / (ms[s] * 1e-3) / 1e9, 1) if nbytes else None})
-    phases = select_phases(c, nat)
     tile_slots = [s for s in range(30) if ms[s] > 0]
     dom = max(tile_slots, key=lambda s: ms[s])
     per_launch_bytes = be * (int(c["prof_in"][dom]) + int(c["prof_out"][dom])) / cnt[dom]
@@ -334,12 +333,11 @@ def profile_step(a, circ, L, nat, BASS, torch, step_ms):
             traffic = tj[nat.SLOT_NAMES[dom]] * per_launch_bytes / be if be == 24 else None
     # the whole simulate call: every gate / rotation / truncation reads its
     # input once and writes its output once (24 B per entry each way), over
-    # the timed step's duration (RDMs, selection, partitions all included)
+    # the timed step's duration (RDMs and barriers included)
     kinds = (0, 1, 2, 4)  # gate1, rot1, gate2, plain; the 2-qubit gate's first pass is overhead
-    step_bytes = be * (sum(int(c["prof_in"][k * 5 + 0]) for k in kinds) +
-                       sum(int(c["prof_out"][k * 5 + 3]) for k in kinds))
+    step_bytes = be * sum(int(c[f][k * 5 + p]) for f in ("prof_in", "prof_out") for k in kinds for p in (0, 2))
     step_gbs = step_bytes / (step_ms * 1e-3) / 1e9
-    top = int(np.argmax(ms))  # the longest kernel overall (the selection has no algorithmic bytes of its own)
+    top = int(np.argmax(ms))  # the longest kernel overall
     roof = {"bound": "hbm", "kernel": nat.SLOT_NAMES[dom], "achieved": round(achieved, 1), "peak": peak,
             "peak_source": peak_src, "unit": "GB/s", "frac": round(achieved / peak, 4),
             "traffic": traffic, "bytes_per_launch": per_launch_bytes,
@@ -353,8 +351,6 @@ def profile_step(a, circ, L, nat, BASS, torch, step_ms):
             "note": "algorithmic bytes = 24 B per entry read + 24 B per entry written; timing from a "
                     "profiled step (CUDA events around each launch on its stream)"}
     kernels = kernels[:12]
-    if phases:
-        kernels.append({"kernel": "k_select_coop phases (us per launch)", **phases})
     return roof, kernels
 
 
@@ -436,9 +432,7 @@ def run_op(a):
         kern.append({"kernel": nat.SLOT_NAMES[sl], "us_per_launch": round(1e3 * ms[sl] / max(cnt[sl], 1), 2),
                      "launches": int(cnt[sl]), "share": round(float(ms[sl] / ms.sum()), 4),
                      "gbs": round(nb / (ms[sl] * 1e-3) / 1e9, 1) if nb else None})
-    phases = select_phases(c, nat)
     print(json.dumps({"op": a.op, "K": K, "n_qubits": n, "dtype": a.dtype, "nnz": st.nnz,
-                      "select_phases_us": phases,
                       "us_per_op": round(1e3 * e0.elapsed_time(e1) / a.steps, 2),
                       "us_per_op_profiled": round(1e3 * ms.sum() / a.steps, 2), "kernels": kern}), flush=True)
 
@@ -643,19 +637,6 @@ def run_form(a):
     torch.cuda.set_device(0)
     fn = {"precision": form_precision, "batched": form_batched, "served": form_served}[a.form]
     print(json.dumps(fn(a, pkg)), flush=True)
-
-
-def select_phases(c, nat):
-    """Mean microseconds per selection launch of each of its phases."""
-    out = {}
-    for sl in nat.SELECT_PHASE_SLOTS:
-        nl = int(c["prof_out"][sl])
-        if nl:
-            out[nat.SLOT_NAMES[sl]] = round(int(c["prof_in"][sl]) / nl / 1e3, 2)
-    nl = int(c["prof_out"][nat.SELECT_SPEC_SLOT])
-    if nl:
-        out["two_level_frac"] = round(int(c["prof_in"][nat.SELECT_SPEC_SLOT]) / nl, 3)
-    return out
 
 
 def over_ranks(dist, dev, seconds, units):

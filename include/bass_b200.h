@@ -74,10 +74,10 @@ typedef struct bass_state {
 } bass_state;
 
 #define BASS_TRACE_WORDS 7 /* u64 per trace event, see bass_ctrl.trace */
-/* Kernel slots of the profiler: 0..29 are the tile kernels (kind * 5 + pass,
-   kind: 0 gate1, 1 rot1, 2 gate2, 3 perm, 4 plain, 5 rdm; pass: 0 evaluation,
-   3 write (the compaction for gate, rotation and truncation kinds), 4 moments;
-   passes 1 and 2 are unused), then 30 partition, 31 selection (one launch),
+/* Kernel slots of the profiler: 0..29 are the op and tile kernels (kind * 5 +
+   pass, kind: 0 gate1, 1 rot1, 2 gate2, 3 perm, 4 plain, 5 rdm; pass: 0 the
+   staged evaluation (rdm: the low-bit pass), 1 its settling, 2 the chip op, 3
+   write, 4 moments), then 30 tile boundaries and sample, 31 workspace clear,
    35 reductions (norm, PR, dot products, the traced rotation commit),
    36 fingerprint, 37 phase2q, 38 phase1q, 39 rdm_final, 40 radix sort,
    41 merge runs, 42 small bookkeeping kernels (dense statevectors among
