@@ -98,7 +98,7 @@ class BASS:
         N = self.N
         for _pass in range(3):
             nat.check(eng.L.bass_rdm_1q(state._cur.ptr, N, nat.ctypes.c_void_p(nat._ptr(eng.rho)), eng.ctrl_ptr,
-                                        eng.ws_ptr, eng.ws_bytes, eng.stream), "bass_rdm_1q")
+                                        eng.ws_ptr, eng.ws_for(state._cur.nmax, 1), eng.stream), "bass_rdm_1q")
             nat.check(eng.L.bass_pr(state._cur.ptr, eng.ctrl_ptr, eng.ws_ptr, eng.ws_bytes, eng.stream), "bass_pr")
             r = eng.rho[:4 * N].cpu().numpy().reshape(N, 4)
             tried = {}

@@ -144,42 +144,44 @@ __host__ __device__ __forceinline__ i128 fx_from(double v) {
 #endif
 }
 
-// floor(v * 2^96) for 0 <= v < 4 as h * 2^48 + l, with h and l integers
-// below 2^50 and 2^48 held exactly in doubles: x = v * 2^96 and the scalings
-// by 2^-48 and 2^48 are exact (powers of two), x - h * 2^48 is exact (both are
-// multiples of ulp(x), the difference is below 2^48), and truncation to an
-// integer rounds nothing else.  Eight such h (or l) add exactly in a double
-// (every partial sum is an integer below 2^53), so a run of terms is summed in
-// floating point and joined into the 128-bit sum once (fx_join96).
-__device__ __forceinline__ void fx_split96(double v, double* h, double* l) {
-  const double x = __dmul_rn(v, 0x1p96);
-  const double hi = trunc(__dmul_rn(x, 0x1p-48));
-  *h = hi;
-  *l = trunc(__dsub_rn(x, __dmul_rn(hi, 0x1p48)));
-}
-__device__ __forceinline__ i128 fx_join96(double h, double l) {
-  return (i128)(((u128)__double2ull_rz(h) << 48) + (u128)__double2ull_rz(l));
-}
-// Signed form: fx_from(v) for |v| < 2 goes to the split accumulators (h, l)
-// (fx_split96 of |v|, negated for v < 0; at most eight terms before
-// fx_join96s), larger values straight to the 128-bit sum w.
+// fx_from(v) for |v| < 2 into split accumulators: |v| is cut at 2^-48 and what
+// is left over at 2^-96 by adding and subtracting a power of two with rounding
+// toward zero (16 + |v| has unit 2^-48, 2^-44 + rest has unit 2^-96), so nothing
+// needs a conversion to an integer (truncating doubles did, at a sixteenth of
+// the rate); eight such h (or l) add exactly in a double, whatever their signs,
+// and are joined into the 128-bit sum once (fx_join96s).  Larger values go
+// straight to the 128-bit sum w.
 __device__ __forceinline__ void fx_acc96(double v, double& h, double& l, i128& w) {
   const double a = fabs(v);
   if (a < 2.0) {
-    double hh, ll;
-    fx_split96(a, &hh, &ll);
-    if (v < 0.0) {
-      hh = -hh;
-      ll = -ll;
-    }
-    h = __dadd_rn(h, hh);
-    l = __dadd_rn(l, ll);
+    const double hh = __dsub_rn(__dadd_rz(a, 16.0), 16.0);
+    const double ll = __dsub_rn(__dadd_rz(__dsub_rn(a, hh), 0x1p-44), 0x1p-44);
+    h = __dadd_rn(h, copysign(hh, v));
+    l = __dadd_rn(l, copysign(ll, v));
   } else {
     w += fx_from(v);
   }
 }
 __device__ __forceinline__ i128 fx_join96s(double h, double l) {
-  return (i128)__double2ll_rz(h) * (i128)281474976710656LL + (i128)__double2ll_rz(l);
+  return (i128)__double2ll_rz(__dmul_rn(h, 0x1p48)) * (i128)281474976710656LL +
+         (i128)__double2ll_rz(__dmul_rn(l, 0x1p96));
+}
+
+// 128-bit sums as four 32-bit limbs, each added into its own 64-bit counter
+// (sums modulo 2^128, so the order of the additions does not matter).
+__device__ __forceinline__ void limb_add(unsigned long long* limb, i128 v) {
+  const u128 u = (u128)v;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const unsigned long long w = (unsigned long long)(u >> (32 * q)) & 0xFFFFFFFFULL;
+    if (w) atomicAdd(limb + q, w);
+  }
+}
+__device__ __forceinline__ i128 limb_get(const unsigned long long* limb) {
+  u128 u = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) u += (u128)limb[q] << (32 * q);
+  return (i128)u;
 }
 
 __device__ __forceinline__ int clz128(u128 u) {

@@ -370,11 +370,19 @@ __device__ __forceinline__ void copy_ragged(E* dst, const E* src, long long lo, 
 // moments of each such qubit (|a|^2 of its bit-0 and bit-1 entries, re and im
 // of a_x conj(a_{x | 2^t})) are the sums of k_tile's P_RDM pass, exact:
 // each warp adds its lanes' sums into its own shared accumulators, and at the
-// end every CTA writes one partial per qubit (slot blockIdx.x of the qubit's
-// set; the grid, at most ws.max_tiles, goes to counter 6 for k_rdm_final).
+// end every CTA adds its sums to the qubits' limbs (rdm_limbs; the workspace
+// clear zeroed them).  Small states take smaller tiles, so that every CTA of the
+// grid has one: what bounds them is the chain of one tile (16,384 entries of 40
+// qubits: 27 us instead of 68 with tiles of kTile).
 constexpr int kRdmSpan = kTile + kRdmHalo;
 constexpr int kRdmSpanPad = kRdmSpan + 2;
 constexpr size_t kRdmLowSmem = (size_t)kRdmSpanPad * (16 + 8);  // amplitudes, keys
+
+// The low-bit pass's sums: four moments of four limbs per qubit, in ws.hist1.
+__device__ __forceinline__ unsigned long long* rdm_limbs(const WsView& ws, int set) {
+  return reinterpret_cast<unsigned long long*>(ws.hist1) + 16 * set;
+}
+static_assert(kMaxSets * 16 * 8 <= kHistBins * 4, "the limbs fit the histogram");
 
 template <bool C64>
 __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ OpArgs a) {
@@ -391,7 +399,10 @@ __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ Op
   for (int i = lane; i < kRdmLowBits * 4; i += 32) sAcc[w][i >> 2][i & 3] = 0;
   const bass_state* in = a.in;
   const long long n = in->nnz;
-  const long long ntiles = plain_tiles(n);
+  long long span = (n + gridDim.x - 1) / gridDim.x;  // entries of a tile: a multiple of kThreads
+  span = span > kTile - kThreads ? kTile : (span + kThreads - 1) / kThreads * kThreads;
+  if (span == 0) span = kThreads;
+  const long long ntiles = (n + span - 1) / span;
   if (tid == 0) mbar_init(&sBar, 1);
   if (tid < kRdmLowBits) {
     int set = -1;
@@ -409,7 +420,7 @@ __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ Op
   // bulk copies need both arrays 16-byte aligned; keys at an 8-byte offset
   // take plain loads
   const bool bulk = ((reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(amps)) & 15) == 0;
-  const bool bad = ntiles > a.ws.max_tiles || (in->amp_type == BASS_AMP_C64) != C64;
+  const bool bad = plain_tiles(n) > a.ws.max_tiles || (in->amp_type == BASS_AMP_C64) != C64;
   if (bad && blockIdx.x == 0 && tid == 0) set_error(a.ctrl, BASS_ERR_WORKSPACE);
   auto amp = [&](int p) {
     const double2 v = C64 ? f2d(sAf[p]) : sA[p];
@@ -423,8 +434,8 @@ __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ Op
     __syncthreads();
     const long long b = sItem;
     if (b >= ntiles) break;
-    const long long lo = b * kTile;  // even: both arrays start on 16-byte words
-    const long long own_end = (lo + kTile < n) ? lo + kTile : n;
+    const long long lo = b * span;  // even: both arrays start on 16-byte words
+    const long long own_end = (lo + span < n) ? lo + span : n;
     const long long hi = (own_end + kRdmHalo < n) ? own_end + kRdmHalo : n;
     const int own = (int)(own_end - lo), E = (int)(hi - lo);
     if (bulk) {
@@ -508,11 +519,9 @@ __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ Op
       i128 sum = 0;
 #pragma unroll
       for (int ww = 0; ww < kThreads / 32; ++ww) sum += sAcc[ww][t][k];
-      a.ws.partials[(long long)set * a.ws.max_tiles + blockIdx.x].s[k] = sum;
+      limb_add(rdm_limbs(a.ws, set) + 4 * k, sum);
     }
   }
-  if (blockIdx.x == 0 && tid == 0)
-    reinterpret_cast<unsigned long long*>(a.ws.counters)[6] = gridDim.x;
 }
 
 // Rotation step, after the write pass: keep the candidate if accepted.
@@ -539,16 +548,16 @@ __global__ void k_commit(bass_state* cur, bass_state* tmp, WsView ws, bass_ctrl*
   }
 }
 
-// low: the sets of qubits at physical bits below kRdmLowBits hold k_rdm_low's
-// partials (one per CTA of its grid, counter 6), the others the merge pass's
-// (one per merge tile)
+// low: the moments of qubits at physical bits below kRdmLowBits are k_rdm_low's
+// limbs, the others the merge pass's partials (one per merge tile)
 __global__ void k_rdm_final(const bass_state* st, double* rho, WsView ws, int first, int low) {
   __shared__ i128 sRed[4 * 8];
   const int set = blockIdx.x;
-  const long long n = st->nnz;
-  const long long ntiles = (low && st->pos[first + set] < kRdmLowBits)
-                               ? (long long)reinterpret_cast<const unsigned long long*>(ws.counters)[6]
-                               : merge_tiles(n);
+  const long long ntiles = merge_tiles(st->nnz);
+  if (low && st->pos[first + set] < kRdmLowBits) {
+    if (threadIdx.x < 4) rho[4 * (first + set) + threadIdx.x] = fx_to(limb_get(rdm_limbs(ws, set) + 4 * threadIdx.x));
+    return;
+  }
   i128 v[4] = {0, 0, 0, 0};
   for (long long t = threadIdx.x; t < ntiles; t += blockDim.x) {
     const Partial& p = ws.partials[(long long)set * ws.max_tiles + t];
@@ -655,7 +664,11 @@ cudaError_t run_rdm(const bass_state* st, int nq, double* rho, bass_ctrl* ctrl, 
   // the partition also clears the small workspace region; the qubits at
   // physical bits below kRdmLowBits take one pass of k_rdm_low instead of a
   // partition and a merge pass each
-  KLAUNCH(S_PARTITION, s, launch_pdl(k_partition, dim3(device().grid_small, nq), dim3(256), 0, s, a, (int)K_RDM, 1));
+  // (no more blocks than the workspace's bound has boundaries, eight to a block:
+  // the full grid for every qubit is 47,000 blocks)
+  const long long want = (ws.max_tiles + 1 + 7) / 8;
+  const int gp = want < device().grid_small ? (int)want : device().grid_small;
+  KLAUNCH(S_PARTITION, s, launch_pdl(k_partition, dim3(gp, nq), dim3(256), 0, s, a, (int)K_RDM, 1));
   if ((e = launch_tile<K_RDM, P_RDM>(a, 0, s, nullptr)) != cudaSuccess) return e;
   {
     static PerDevice grid_c64, grid_c128;
@@ -663,7 +676,6 @@ cudaError_t run_rdm(const bass_state* st, int nq, double* rho, bass_ctrl* ctrl, 
     if ((e = c64 ? smem_grid(grid_c64, k_rdm_low<true>, kRdmLowSmem, &gl)
                  : smem_grid(grid_c128, k_rdm_low<false>, kRdmLowSmem, &gl)) != cudaSuccess)
       return e;
-    if (gl > ws.max_tiles) gl = (int)ws.max_tiles;  // one partial slot per CTA
     a.counter = 5;
     a.prof = prof_on() ? 1 : 0;
     if (c64)

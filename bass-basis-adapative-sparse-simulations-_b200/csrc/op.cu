@@ -153,23 +153,6 @@ __device__ __forceinline__ int op_exit(bass_ctrl* c, int nblk, bool failed) {
 // ---------------------------------------------------------------------------
 // exact sums
 // ---------------------------------------------------------------------------
-// 128-bit sums as four 32-bit limbs, each added into its own 64-bit counter
-// (sums modulo 2^128, so the order of the additions does not matter).
-__device__ __forceinline__ void limb_add(unsigned long long* limb, i128 v) {
-  const u128 u = (u128)v;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const unsigned long long w = (unsigned long long)(u >> (32 * q)) & 0xFFFFFFFFULL;
-    if (w) atomicAdd(limb + q, w);
-  }
-}
-__device__ __forceinline__ i128 limb_get(const unsigned long long* limb) {
-  u128 u = 0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) u += (u128)limb[q] << (32 * q);
-  return (i128)u;
-}
-
 // Sums of fx_from(p) over terms 0 <= p < 1: the sum is carried in two doubles
 // that stay within one binade, h in [16, 32) with unit 2^-48 and l in
 // [2^-44, 2^-43) with unit 2^-96, and every addition rounds toward zero: h + p
