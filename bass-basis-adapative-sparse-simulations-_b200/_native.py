@@ -215,15 +215,17 @@ class Engine:
     # -- plumbing ---------------------------------------------------------------
     @property
     def stream(self):
-        return ctypes.c_void_p(self.torch.cuda.current_stream(self.device).cuda_stream)
+        # the current stream's handle as an integer: the Stream object that
+        # torch.cuda.current_stream builds costs 7 us a call, more than a small op
+        return self.torch._C._cuda_getCurrentRawStream(self.device.index)
 
     @property
     def ctrl_ptr(self):
-        return ctypes.c_void_p(_ptr(self.ctrl))
+        return self.ctrl.data_ptr()
 
     @property
     def ws_ptr(self):
-        return ctypes.c_void_p(_ptr(self.ws))
+        return self.ws.data_ptr()
 
     def ws_for(self, entries, slots):
         """The workspace size to pass for an op on at most ``entries`` entries
@@ -329,7 +331,7 @@ class DevState:
 
     @property
     def ptr(self):
-        return ctypes.c_void_p(_ptr(self.desc))
+        return self.desc.data_ptr()
 
     def init(self, key: int = 0):
         check(self.eng.L.bass_state_init_typed(self.ptr, ctypes.c_void_p(_ptr(self.keys)),
