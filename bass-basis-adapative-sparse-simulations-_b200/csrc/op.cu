@@ -31,7 +31,7 @@
 // evaluation of every child into 56 bytes of staging per entry, a selection of
 // three histogram passes with grid barriers, and compaction):
 //   n              64   508  16384  65536  300000   2^20   2^22
-//   1-qubit gate   16    16     35     42      65     86    200
+//   1-qubit gate   16    16     35     42      65     86    194
 //   before         41    45     63     66      80    108    224
 //   2-qubit gate   26    36     53     66     101    140    308
 //   before         57    62    104    120     135    184    447
@@ -1630,7 +1630,9 @@ __device__ __forceinline__ void staged_final(const OpArgs& a, OpSh& sh, const Op
 // The write: every region's survivors, copied to their place, one region per
 // warp and round.  Where they go: the tile's offset plus what the tile's
 // earlier regions keep (its eight counts are one 16-byte load), so warps need
-// no barrier.
+// no barrier.  Staged children are read and survivors written once: streaming
+// accesses (202 -> 194 us per gate at 2^22 entries for the stores).  Four loads in
+// flight per lane at four blocks per SM; two (206 us) or eight (225) are slower.
 template <int KIND, bool C64>
 __device__ __forceinline__ void staged_write(const OpArgs& a, const Grp& g, OpSh& sh, const OpCtx& X) {
   constexpr int NS = slots_per_entry(KIND);
@@ -1693,9 +1695,9 @@ __device__ __forceinline__ void staged_write(const OpArgs& a, const Grp& g, OpSh
         const int ob = __shfl_sync(0xffffffffu, inc - pc, (l0 + u) & 31);
         if ((mw[u] >> lane) & 1u) {
           const long long o = o0 + ob + __popc(mw[u] & lt);
-          okeys[o] = kk[u];
-          if (C64) oampf[o] = af[u];
-          else oamps[o] = aa[u];
+          __stcs(okeys + o, kk[u]);
+          if (C64) __stcs(oampf + o, af[u]);
+          else __stcs(oamps + o, aa[u]);
         }
       }
     }
