@@ -312,7 +312,7 @@ int bass_merge_sorted(uint64_t* keys, double* amps, int64_t n, int64_t* n_out, v
    calls above: the host array describes the segments, the library copies it
    into the batch workspace (bass_batch_ws_bytes) and launches once per pass
    for all of them.  All states of one call must have the same amplitude type;
-   n <= 256 for ops that truncate or rotate (their selection keeps every block
+   n <= bass_batch_max_segments() (an op's grid barriers keep every block
    of the grid resident).  No counterpart in the reference, whose simulators
    run one state at a time. */
 typedef struct bass_seg_op {
