@@ -2032,7 +2032,9 @@ static cudaError_t merge_op_seg(const OpArgs* ops, int nseg, SegPlan* plan, cuda
   int grid = 0;
   cudaError_t e = seg_op_grid<KIND, C64>(&grid);
   if (e != cudaSuccess) return e;
-  if (nseg > grid) return cudaErrorInvalidValue;  // the groups' barriers need every block resident
+  int most = grid;  // the groups' barriers need every block resident
+  if (KIND != K_PERM && (e = seg_max_segments(&most)) != cudaSuccess) return e;
+  if (nseg > most) return cudaErrorInvalidValue;
   if ((e = run_seg_plan(ops, nseg, KIND, plan, s)) != cudaSuccess) return e;
   KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op_seg<KIND, C64>, dim3(grid), dim3(kThreads), kFusedSmem, s, ops,
                                                 (const SegPlan*)plan));
