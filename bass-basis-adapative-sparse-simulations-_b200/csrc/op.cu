@@ -1805,6 +1805,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_op(const __grid_constant__ OpAr
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const SegPlan* plan) {
   __shared__ OpArgs sa;
+  pdl_wait();  // the plan is the kernel before's
   const Grp g = seg_enter(ops, plan, &sa, nullptr);
   op_body<KIND, C64, true>(sa, g);
 }
