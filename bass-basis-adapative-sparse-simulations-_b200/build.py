@@ -11,13 +11,15 @@ import glob
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libbass_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-         "-fmad=false", "-Xcompiler", "-fPIC", "-shared", "-Xptxas", "-O3"]
+ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC", "-Xptxas", "-O3"]
 
 
 def sources():
@@ -34,8 +36,14 @@ def build(force=False, verbose=False):
         t = os.path.getmtime(LIB)
         if all(os.path.getmtime(d) <= t for d in deps()):
             return LIB
-    cmd = [NVCC] + FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB] + sources()
-    subprocess.check_call(cmd)
+    # a compiler per source file, side by side: the op kernels are a file per
+    # kind, since together they take two minutes
+    flags = FLAGS + (["-Xptxas", "-v"] if verbose else [])
+    with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        objs = [os.path.join(tmp, os.path.basename(s)[:-3] + ".o") for s in sources()]
+        list(pool.map(lambda so: subprocess.check_call([NVCC] + flags + ["-c", so[0], "-o", so[1]]),
+                      zip(sources(), objs)))
+        subprocess.check_call([NVCC] + ARCH + ["-shared", "-o", LIB] + objs)
     return LIB
 
 

@@ -611,7 +611,7 @@ struct WsView {
   unsigned int* hist1;           // kHistBins bins
   unsigned int* hist2;           // kHistBins bins
   Partial* partials;             // kMaxSets x max_tiles
-  // the staged route's children, per region of a tile (op.cu), and scratch of others
+  // the staged route's children, per region of a tile (op.cuh), and scratch of others
   unsigned long long* cand_bits; // |a|^2 patterns of the undecided children
   unsigned long long* cand_key;  // their places (16 bits each); the sort's index buffers
   SelState* sel;
