@@ -16,6 +16,8 @@
 // moves took 6.4 ms (150,001 complex64 entries of 30 bits: 0.10 and 0.22 ms).
 // Up to kSortTile entries are sorted by one CTA without leaving shared memory:
 // 19 us instead of 65 at 256 entries of 12 bits.
+#include <math.h>
+
 #include "internal.h"
 
 namespace bass {
@@ -26,6 +28,7 @@ constexpr int kSortItems = 8;                          // per thread
 constexpr int kSortTile = kSortThreads * kSortItems;   // 4096
 constexpr int kDigits = 256;
 constexpr int kMaxPasses = 8;
+constexpr int kSortCounters = kMaxPasses + 2;
 
 struct SortArgs {
   const bass_state* st;      // export: the source state (n = its nnz), or nullptr
@@ -38,7 +41,7 @@ struct SortArgs {
   unsigned int* idx0;        // index buffers
   unsigned int* idx1;
   unsigned int* hist;        // kMaxPasses x kDigits counts, zeroed before the launch
-  unsigned long long* ctr;   // zeroed: [p] tile counter of pass p, [kMaxPasses] barrier arrivals
+  unsigned long long* ctr;   // zeroed: [p] tile counter of pass p, [kMaxPasses] barrier arrivals, [kMaxPasses + 1] give-ups
   unsigned long long* status;  // per tile and digit: pass tag and count, see look_back
   long long max_n;
   long long max_tiles;       // tiles the status array holds
@@ -56,6 +59,7 @@ __device__ __forceinline__ unsigned long long sort_word(int pass, int flag, unsi
 
 __device__ __forceinline__ void sort_error(const SortArgs& a) {
   if (a.ctrl) set_error(a.ctrl, BASS_ERR_WAIT);
+  else atomicAdd(a.ctr + kMaxPasses + 1, 1ULL);
 }
 
 // Barrier of the launch's nblk working blocks (all resident: a cooperative
@@ -231,7 +235,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(const __grid_constant_
   const uint64_t* in = a.st ? a.st->keys : a.keys;
   auto first_key = [&](long long i) { return a.st ? true_key(in[i], qat, 64) : in[i]; };
   __syncthreads();
-  const long long lim = kSpinLimit;
+  const long long lim = a.ctrl ? wait_limit(a.ctrl) : kSpinLimit;
 
   if (ntiles == 1) {
     // one tile: every pass in block 0's shared memory
@@ -343,6 +347,17 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(const __grid_constant_
   }
 }
 
+// After a sort without a control block: a give-up leaves keys out of place and
+// nothing else would say so, so every amplitude of the result becomes NaN.
+__global__ void k_sort_check(SortArgs a, int c64) {
+  if (a.ctr[kMaxPasses + 1] == 0ULL) return;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < 2 * a.n_host; i += step) {
+    if (c64) static_cast<float*>(a.amps)[i] = NAN;
+    else static_cast<double*>(a.amps)[i] = NAN;
+  }
+}
+
 template <typename P>
 static cudaError_t launch_sort(SortArgs a, const WsView& ws, cudaStream_t s) {
   static PerDevice cache;
@@ -362,8 +377,8 @@ static cudaError_t launch_sort(SortArgs a, const WsView& ws, cudaStream_t s) {
   // the digit histograms and counters share the selection's histogram area
   a.hist = ws.hist1;
   a.ctr = reinterpret_cast<unsigned long long*>(ws.hist1 + kMaxPasses * kDigits);
-  static_assert(kMaxPasses * kDigits + 2 * (kMaxPasses + 1) <= kHistBins, "sort counters fit the histogram area");
-  e = cudaMemsetAsync(a.hist, 0, (kMaxPasses * kDigits + 2 * (kMaxPasses + 1)) * sizeof(unsigned int), s);
+  static_assert(kMaxPasses * kDigits + 2 * kSortCounters <= kHistBins, "sort counters fit the histogram area");
+  e = cudaMemsetAsync(a.hist, 0, (kMaxPasses * kDigits + 2 * kSortCounters) * sizeof(unsigned int), s);
   if (e != cudaSuccess) return e;
   a.tkeys = ws.tmp_keys;
   a.idx0 = reinterpret_cast<unsigned int*>(ws.cand_key);
@@ -374,6 +389,10 @@ static cudaError_t launch_sort(SortArgs a, const WsView& ws, cudaStream_t s) {
   void* args[] = {&a};
   KLAUNCH(S_SORT, s, e = cudaLaunchCooperativeKernel((const void*)k_sort<P>, dim3(grid), dim3(kSortThreads), args,
                                                      smem, s));
+  if (e == cudaSuccess && !a.ctrl) {
+    KLAUNCH(S_SORT, s, k_sort_check<<<device().sms, 256, 0, s>>>(a, sizeof(P) == 8));
+    e = cudaGetLastError();
+  }
   return e;
 }
 

@@ -295,7 +295,9 @@ int bass_fingerprint(const bass_state* st, double pmin, uint64_t* out6, void* ws
 
 /* ---- array-level kernels (the reference's Numba kernels on plain arrays) --- */
 /* sparse_state.py:150-172 radix_sort_uint64: stable sort of n (key, amp) pairs
-   on the low key_bits bits; in place (uses the workspace). */
+   on the low key_bits bits; in place (uses the workspace).  A
+   bounded wait of the sort that gives up sets BASS_ERR_WAIT in ctrl; with
+   ctrl NULL it makes every amplitude NaN instead. */
 int bass_radix_sort_u64(uint64_t* keys, double* amps, int64_t n, int key_bits, void* ws,
                         size_t ws_bytes, bass_ctrl* ctrl, void* stream);
 /* sparse_state.py:127-147 merge_sorted_kernel: merge adjacent equal keys of a
