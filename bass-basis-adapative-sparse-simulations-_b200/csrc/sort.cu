@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(const __grid_constant_
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const long long n = a.n_dev ? *a.n_dev : a.n_host;
   const long long ntiles = (n + kSortTile - 1) / kSortTile;
-  if (n <= 0 || n > a.max_n || ntiles > a.max_tiles) return;
+  if (n > a.max_n || ntiles > a.max_tiles) return;
   double r0 = 1.0, r1 = 1.0;
   if (a.st) {
     if (a.st->amp_type != a.amp_type) {
@@ -231,6 +231,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(const __grid_constant_
     r0 = a.st->rscale[0];
     r1 = a.st->rscale[1];
   }
+  if (n <= 0) return;
   const bool c64 = sizeof(P) == 8;
   const uint64_t* in = a.st ? a.st->keys : a.keys;
   auto first_key = [&](long long i) { return a.st ? true_key(in[i], qat, 64) : in[i]; };
