@@ -1712,11 +1712,13 @@ __device__ __forceinline__ void staged_write(const OpArgs& a, const Grp& g, OpSh
 __device__ __forceinline__ void prof_add(int64_t* slots, int slot, long long v) {
   atomicAdd(reinterpret_cast<unsigned long long*>(slots + slot), (unsigned long long)v);
 }
-// The op's last block: the result, its bookkeeping and profile counts.
-__device__ __forceinline__ void op_close(const OpArgs& a, int kind, int pass, const OpResult& R, long long n) {
+// The op's last block: the result, its bookkeeping and profile counts (pass_in:
+// the kernel that read the entries, pass_out: the one that wrote the survivors).
+__device__ __forceinline__ void op_close(const OpArgs& a, int kind, int pass_in, int pass_out, const OpResult& R,
+                                         long long n) {
   if (a.prof && threadIdx.x == 0) {
-    prof_add(a.ctrl->prof_in, kind * 5 + pass, n);
-    if (!R.skip) prof_add(a.ctrl->prof_out, kind * 5 + pass, R.n_written);
+    prof_add(a.ctrl->prof_in, kind * 5 + pass_in, n);
+    if (!R.skip) prof_add(a.ctrl->prof_out, kind * 5 + pass_out, R.n_written);
   }
   __syncthreads();
   op_finalize(a, kind, R);
@@ -1791,7 +1793,7 @@ __device__ __forceinline__ void op_body(const OpArgs& a, Grp g) {
   }
   pdl_trigger();
   // every block knows the result; the last one out only resets the barrier
-  if (g.bid == 0 && ok) op_close(a, KIND, P_GATHER, sh.R, n);
+  if (g.bid == 0 && ok) op_close(a, KIND, P_GATHER, P_GATHER, sh.R, n);
   if (g.nblk > 1) op_exit(a.ctrl, g.nblk, !ok);
 }
 
@@ -1855,7 +1857,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_eval(const __grid_constant__
     if (threadIdx.x == 0) sh.R = OpResult{};
     if (!X.bad) ok = staged_perm<C64>(a, sh, X, &phase, smem);
     pdl_trigger();
-    if (op_exit(a.ctrl, gridDim.x, !ok) == 1) op_close(a, KIND, P_HIST, sh.R, X.S.n);
+    if (op_exit(a.ctrl, gridDim.x, !ok) == 1) op_close(a, KIND, P_HIST, P_HIST, sh.R, X.S.n);
     return;
   }
   load_words(a, kStageAt, sh.St);
@@ -1917,7 +1919,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_write(const __grid_constant_
   __syncthreads();
   if (!X.bad && !sh.R.failed) staged_write<KIND, C64>(a, whole_grid(), sh, X);
   pdl_trigger();
-  if (op_exit(a.ctrl, gridDim.x, sh.R.failed != 0) == 1) op_close(a, KIND, P_HIST, sh.R, X.S.n);
+  if (op_exit(a.ctrl, gridDim.x, sh.R.failed != 0) == 1) op_close(a, KIND, P_HIST, P_WRITE, sh.R, X.S.n);
 }
 
 // ---------------------------------------------------------------------------

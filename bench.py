@@ -330,12 +330,15 @@ def profile_step(a, circ, L, nat, BASS, torch, step_ms):
     if os.path.exists(tfile):
         tj = json.load(open(tfile))
         if nat.SLOT_NAMES[dom] in tj:
-            traffic = tj[nat.SLOT_NAMES[dom]] * per_launch_bytes / be if be == 24 else None
+            # the file's figure is per entry that the kernel reads
+            traffic = tj[nat.SLOT_NAMES[dom]] * int(c["prof_in"][dom]) / cnt[dom] if be == 24 else None
     # the whole simulate call: every gate / rotation / truncation reads its
     # input once and writes its output once (24 B per entry each way), over
     # the timed step's duration (RDMs and barriers included)
     kinds = (0, 1, 2, 4)  # gate1, rot1, gate2, plain; the 2-qubit gate's first pass is overhead
-    step_bytes = be * sum(int(c[f][k * 5 + p]) for f in ("prof_in", "prof_out") for k in kinds for p in (0, 2))
+    # (the staged route reads in its evaluation, 0, and writes in its last pass, 3; the chip op, 2, does both)
+    step_bytes = be * sum(int(c[f][k * 5 + p]) for f, ps in (("prof_in", (0, 2)), ("prof_out", (2, 3)))
+                          for k in kinds for p in ps)
     step_gbs = step_bytes / (step_ms * 1e-3) / 1e9
     top = int(np.argmax(ms))  # the longest kernel overall
     roof = {"bound": "hbm", "kernel": nat.SLOT_NAMES[dom], "achieved": round(achieved, 1), "peak": peak,
@@ -348,8 +351,9 @@ def profile_step(a, circ, L, nat, BASS, torch, step_ms):
             "longest_kernel": {"kernel": nat.SLOT_NAMES[top], "share": round(float(ms[top] / ms.sum()), 4),
                                "note": "share of the profiled step; the roofline above is that of the "
                                        "longest tile pass, the kernels that move the state's own bytes"},
-            "note": "algorithmic bytes = 24 B per entry read + 24 B per entry written; timing from a "
-                    "profiled step (CUDA events around each launch on its stream)"}
+            "note": "algorithmic bytes = 24 B per state entry that the kernel reads or writes (a staged "
+                    "evaluation reads, the write pass after it writes); timing from a profiled step "
+                    "(CUDA events around each launch on its stream)"}
     kernels = kernels[:12]
     return roof, kernels
 
