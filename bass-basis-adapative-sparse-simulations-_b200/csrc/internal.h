@@ -32,6 +32,7 @@ struct OpArgs {
   int guard;      // K_IDENT: run only if ws.sel->pad (zero flag) is set
   int prof;       // count entries into ctrl->prof_in / prof_out
   int fin_mode;   // 0 gate / truncation, 1 rotation step
+  int staged;     // launches of the staged route follow the first one
   int commit;     // rotation step: the op also commits (swaps in an accepted candidate)
   int j;          // rotation step: the rotated qubit
   long long k_cond, k_keep;

@@ -57,6 +57,11 @@ constexpr int kSamples = 16384;                  // sampled entries of the brack
 constexpr int kSampleMargin = 512;               // 4 sqrt(kSamples): ranks around the estimate
 constexpr int kRegion = 32 * kPerThread;         // Z positions of a warp's region of a tile
 constexpr int kRegions = kThreads / 32;          // regions of a tile
+// Blocks of a staged op's first launch: they do the whole op for a state of up
+// to kFirstBlocks x kChipStep = 32,512 entries under a larger bound.  One per SM
+// (148) would take states of 75,000 entries, but costs every op at 2^22 entries
+// 3 us (202 instead of 199), and at 65,536 entries the staged route is as fast.
+constexpr int kFirstBlocks = 64;
 // |a|^2 bins of the sample: 128 per power of two over [2^-64, 1)
 constexpr int kSampleBase = (1023 - 64) << 7;
 
@@ -78,15 +83,27 @@ constexpr size_t kChipSmem = kChipHistAt + (size_t)kChipBins * 4;
 // grid barriers
 // ---------------------------------------------------------------------------
 // One word of the control block (zero between ops): bits 0-19 arrivals of the
-// op's barriers, bits 20-30 blocks that are done, bit 31 some block gave up.
-// The last block to finish resets it.
-constexpr unsigned kArriveMask = (1u << 20) - 1, kExitOne = 1u << 20, kFailBit = 1u << 31;
+// op's barriers, bits 20-29 blocks that are done, bit 30 the launch was called
+// off, bit 31 some block gave up.  The last block to finish resets it.
+//
+// Blocks that wait for one another have to be resident together: their launch
+// is cooperative, or its first barrier may be called off.  A cooperative launch
+// does not start beside the end of the kernel before it (4 us of every staged
+// op at 2^20 entries), so the launch that only does the whole op for states
+// that turn out small is a plain one: whoever waits too long at its first
+// barrier calls the launch off, which nobody can once all blocks have arrived
+// (and so are resident), and the staged launches that follow do the op.
+constexpr unsigned kArriveMask = (1u << 20) - 1, kExitOne = 1u << 20, kExitMask = (1u << 10) - 1;
+constexpr unsigned kOffBit = 1u << 30, kFailBit = 1u << 31;
+constexpr long long kOffSpins = 512;  // polls (some 100 us) before a launch is called off
 
 struct Gate {
   unsigned* word;
   int nact;         // blocks that take part
   int all;          // arrivals of the first barrier (every block of the launch may count there)
+  int may_off;      // the first barrier may be called off
   unsigned passed;  // barriers entered
+  bool off;         // it was
 };
 
 // Block-wide: arrive (everything written before is visible to the blocks that
@@ -100,31 +117,42 @@ __device__ __forceinline__ void gate_arrive(Gate& b) {
   }
 }
 // Block-wide: wait until every block has arrived (bounded; false on give-up,
-// with BASS_ERR_WAIT recorded).
-__device__ __forceinline__ bool gate_wait(const Gate& b, bass_ctrl* c) {
-  __shared__ int sOk;
+// with BASS_ERR_WAIT recorded, and when the launch is called off).
+__device__ __forceinline__ bool gate_wait(Gate& b, bass_ctrl* c) {
+  __shared__ int sOk;  // 1 all arrived, 0 gave up, -1 called off
   if (b.nact > 1 || (b.passed == 1 && b.all > 1)) {
     if (threadIdx.x == 0) {
       const unsigned target = (unsigned)b.all + (b.passed - 1) * (unsigned)b.nact;
-      const long long lim = wait_limit(c);
+      const bool may_off = b.may_off && b.passed == 1;
+      long long lim = wait_limit(c);
+      if (may_off && lim > kOffSpins) lim = kOffSpins;
       long long spins = 0;
       int ok = 1;
       for (;;) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(b.word) : "memory");
-        if ((v & kArriveMask) >= target) break;
-        if (++spins > lim) {
-          set_error(c, BASS_ERR_WAIT);
-          ok = 0;
+        if (may_off && (v & kOffBit)) {
+          ok = -1;
           break;
         }
-        __nanosleep(b.nact > 64 ? 100 : 20);  // (hundreds of pollers would hold up the arrivals)
+        if ((v & kArriveMask) >= target) break;
+        if (++spins > lim) {
+          if (!may_off) {
+            set_error(c, BASS_ERR_WAIT);
+            ok = 0;
+            break;
+          }
+          atomicCAS(b.word, v, v | kOffBit);  // (or the word has changed: look again)
+        } else {
+          __nanosleep(b.nact > 64 ? 100 : 20);  // (hundreds of pollers would hold up the arrivals)
+        }
       }
       __threadfence();
       sOk = ok;
     }
     __syncthreads();
-    return sOk != 0;
+    b.off = sOk < 0;
+    return sOk > 0;
   }
   __syncthreads();
   return true;
@@ -133,8 +161,8 @@ __device__ __forceinline__ bool gate_sync(Gate& b, bass_ctrl* c) {
   gate_arrive(b);
   return gate_wait(b, c);
 }
-// Block-wide, once per block of the group: 1 in the last block to call (2 if
-// some block gave up), 0 in the others.
+// Block-wide, once per block of the group, in the last block to call: 1, or 2
+// if some block gave up, or 3 if the launch was called off; 0 in the others.
 __device__ __forceinline__ int op_exit(bass_ctrl* c, int nblk, bool failed) {
   __shared__ int sLast;
   __syncthreads();
@@ -143,8 +171,8 @@ __device__ __forceinline__ int op_exit(bass_ctrl* c, int nblk, bool failed) {
     if (failed) atomicOr(&c->sync_counter, kFailBit);
     __threadfence();
     const unsigned old = atomicAdd(&c->sync_counter, kExitOne);
-    const bool last = ((old >> 20) & 0x7FFu) == (unsigned)(nblk - 1);
-    sLast = last ? ((old & kFailBit) ? 2 : 1) : 0;
+    const bool last = ((old >> 20) & kExitMask) == (unsigned)(nblk - 1);
+    sLast = last ? ((old & kFailBit) ? 2 : (old & kOffBit) ? 3 : 1) : 0;
     if (last) *(volatile uint32_t*)&c->sync_counter = 0u;
     __threadfence();
   }
@@ -386,8 +414,9 @@ struct OpResult {
   double kept, total, pr_new;
   int trunc, accept;
   int skip;    // a rejected rotation candidate is not written
-  int failed;  // a wait gave up: no result
+  int failed;  // a wait gave up: no result (or kOver)
 };
+constexpr int kOver = 2;  // the op's first launch did the whole op, or refused it
 
 // What a candidate's PR has to stay below (bass_simulator.py:795-814, with the
 // relative tolerance).  Read before the first barrier: the op's end rewrites pr_cur.
@@ -520,8 +549,10 @@ struct OpStage {
   Cut cut;
   long long n_out;
   int trunc;
-  int state;  // 0 the bracket holds the threshold, 1 it missed, 2 a wait gave up
+  int state;  // StageState
 };
+enum StageState { ST_OK = 0, ST_MISSED = 1 /* the threshold is outside the bracket */, ST_GAVE_UP = 2,
+                  ST_OVER = 3 /* as kOver */ };
 static_assert(sizeof(OpResult) % 8 == 0 && sizeof(OpResult) <= 8 * (kStageAt - kResultAt), "result words");
 static_assert(sizeof(OpStage) % 8 == 0 && sizeof(OpStage) <= 8 * (kListAt - kStageAt), "stage words");
 
@@ -566,6 +597,14 @@ __device__ __forceinline__ void load_words(const OpArgs& a, int at, T& v) {
         __ldcg(reinterpret_cast<const unsigned long long*>(a.ws.red) + at + threadIdx.x);
 }
 
+__device__ __forceinline__ OpStage* stage_of(const OpArgs& a) {
+  return reinterpret_cast<OpStage*>(reinterpret_cast<unsigned long long*>(a.ws.red) + kStageAt);
+}
+__device__ __forceinline__ OpResult* result_of(const OpArgs& a) {
+  return reinterpret_cast<OpResult*>(reinterpret_cast<unsigned long long*>(a.ws.red) + kResultAt);
+}
+
+constexpr long long kMaxEntries = 1LL << 31;  // an op takes fewer
 // The op's input, the same in every thread.
 struct OpCtx {
   TileSrc S;
@@ -594,7 +633,7 @@ __device__ __forceinline__ OpCtx op_ctx(const OpArgs& a) {
   X.may_trunc = KIND != K_PERM && a.k_cond >= 0 && children > a.k_cond && children > a.k_keep;
   X.ntiles = KIND == K_IDENT ? plain_tiles(n) : merge_tiles(n);
   X.bad = (in->amp_type == BASS_AMP_C64) != C64 || X.ntiles > a.ws.max_tiles || children > a.ws.max_n ||
-          n >= (1LL << 31);
+          n >= kMaxEntries;
   return X;
 }
 // One thread: the refusal's error bits.
@@ -1054,19 +1093,18 @@ __device__ __forceinline__ void sample_entry(const OpArgs& a, const OpCtx& X, lo
   }
 }
 
+__device__ __forceinline__ bool is_bracketed(const OpArgs& a, const OpCtx& X) { return X.may_trunc && a.k_keep > 0; }
 
 // Clears the counters, both histograms and the tiles' counts.
-__device__ __forceinline__ void staged_zero(const OpArgs& a, const Grp& g, const OpCtx& X) {
+__device__ __forceinline__ void staged_zero(const OpArgs& a, const Grp& g, long long ntiles) {
   const long long gthreads = (long long)g.nblk * kThreads, gtid = (long long)g.bid * kThreads + threadIdx.x;
   for (long long i = gtid; i < kHistBins / 4; i += gthreads) {
     reinterpret_cast<uint4*>(a.ws.hist1)[i] = make_uint4(0, 0, 0, 0);
     reinterpret_cast<uint4*>(a.ws.hist2)[i] = make_uint4(0, 0, 0, 0);
   }
-  for (long long i = gtid; i < X.ntiles; i += gthreads) a.ws.status[i] = 0ULL;
+  for (long long i = gtid; i < ntiles; i += gthreads) a.ws.status[i] = 0ULL;
   if (gtid < kOpCounters) reinterpret_cast<unsigned long long*>(a.ws.counters)[gtid] = 0ULL;
 }
-
-__device__ __forceinline__ bool is_bracketed(const OpArgs& a, const OpCtx& X) { return X.may_trunc && a.k_keep > 0; }
 
 // Tile boundaries, one warp each from the front of the grid, and the sample's
 // histogram, eight lanes per entry from its end (both are chains of dependent
@@ -1339,12 +1377,12 @@ __device__ __forceinline__ void staged_plan(const OpArgs& a, OpSh& sh, const OpC
   const long long n_staged = (long long)*(const volatile unsigned long long*)(cn + C_STAGED);
   const int trunc = X.may_trunc && !(n_out <= a.k_cond || a.k_keep >= n_out);
   Cut cut{0ULL, 0ULL, 0ULL, 0, CUT_ALL, 0, 0};
-  int state = 0;
+  int state = ST_OK;
   Bracket Bn = B;
   if (trunc && a.k_keep <= 0) {
     cut.mode = CUT_NONE;
   } else if (!(trunc ? (n_def <= a.k_keep && n_staged >= a.k_keep) : n_staged == n_out)) {
-    state = 1;
+    state = ST_MISSED;
   } else if (trunc) {
     cut.mode = CUT_BITS;
     cut.lo = B.lo;
@@ -1428,7 +1466,7 @@ __device__ __forceinline__ void visit_regions(const OpArgs& a, const Grp& g, lon
 
 // The undecided children's threshold, found and applied: masks, counts per tile,
 // sums, and the list of the (at most kSelMax) children still to be ranked.  All
-// blocks of the launch resident.  A bracket that missed (sh.St.state 1) is
+// blocks of the launch resident.  A bracket that missed (ST_MISSED) is
 // replaced first.  False on a give-up.
 template <int KIND, bool C64>
 __device__ __forceinline__ bool staged_settle(const OpArgs& a, const Grp& g, OpSh& sh, const OpCtx& X, Gate& gate,
@@ -1443,7 +1481,7 @@ __device__ __forceinline__ bool staged_settle(const OpArgs& a, const Grp& g, OpS
   auto clear = [&](unsigned* h) {
     for (long long i = gtid; i < kHistBins / 4; i += gthreads) reinterpret_cast<uint4*>(h)[i] = make_uint4(0, 0, 0, 0);
   };
-  if (sh.St.state == 1) {
+  if (sh.St.state == ST_MISSED) {
     // the exact bracket, from the histogram of all children, and the
     // evaluation again
     clear(a.ws.hist1);
@@ -1730,7 +1768,7 @@ template <int KIND, bool C64>
 __device__ __forceinline__ bool op_staged(const OpArgs& a, const Grp& g, OpSh& sh, const OpCtx& X, Gate& gate,
                                           unsigned char* smem) {
   unsigned phase = 0;
-  staged_zero(a, g, X);
+  staged_zero(a, g, X.ntiles);
   if (!gate_sync(gate, a.ctrl)) return false;
   staged_prep<KIND, C64>(a, g, X);
   if (!gate_sync(gate, a.ctrl)) return false;
@@ -1755,87 +1793,92 @@ __device__ __forceinline__ bool op_staged(const OpArgs& a, const Grp& g, OpSh& s
   }
 }
 
-// One op on the blocks of a group: the chip route if they can hold the state,
-// the staged route otherwise (STAGED: compiled in).
-template <int KIND, bool C64, bool STAGED>
-__device__ __forceinline__ void op_body(const OpArgs& a, Grp g) {
+// The first launch of an op: the whole op on the chip route if the group's
+// blocks can hold the state, otherwise (a.staged) the staged route's clearing.
+// The later launches of an op that is over return at once.
+template <int KIND, bool C64, bool FUSED>
+__device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ OpSh sh;
   const int tid = threadIdx.x;
+  if (!FUSED && a.staged) {
+    // too large for the chip route and accepted: as little code as can be (its
+    // lines come from DRAM after an op on a large state)
+    const long long n = a.in->nnz, nt = KIND == K_IDENT ? plain_tiles(n) : merge_tiles(n);
+    if (n > (long long)g.nblk * kChipStep && n * slots_per_entry(KIND) <= a.ws.max_n && nt <= a.ws.max_tiles &&
+        n < kMaxEntries && (a.in->amp_type == BASS_AMP_C64) == C64) {
+      pdl_trigger();
+      staged_zero(a, g, nt);
+      if (g.bid == 0 && tid == 0) stage_of(a)->state = ST_OK;
+      return;
+    }
+  }
   const OpCtx X = op_ctx<KIND, C64>(a);
   const long long n = X.S.n;
+  const int step = X.bad ? 0 : chip_step(n, g.nblk);
   if (tid == 0) mbar_init(&sh.bar, 1);
   out_order_par(a.in, KIND, a.q, a.gb, sh.qat);
   __syncthreads();
   if (tid == 0) op_preload(a, sh);
   __syncthreads();
-  bool ok = true;
+  bool ok = true, off = false;
   unsigned* word = reinterpret_cast<unsigned*>(&a.ctrl->sync_counter);
-  const int step = chip_step(n, g.nblk);
-  if (X.bad || (step == 0 && !STAGED)) {
-    if (tid == 0) sh.R = OpResult{};
-    if (g.bid == 0 && tid == 0) op_refuse(a, C64);
-    // block 0 closes the op below: the others must have read its descriptors
-    Gate gate{word, 1, g.nblk, 0u};
-    gate_arrive(gate);
-    if (g.bid == 0) ok = gate_wait(gate, a.ctrl);
-  } else if (step) {
+  if (step) {
     // every block counts at the first barrier (it has then read the
     // descriptors, which block 0 rewrites at the end), the ones with a tile
     // at the others
     const int nact = n > 0 ? (int)((n + step - 1) / step) : 1;
-    Gate gate{word, nact, g.nblk, 0u};
+    Gate gate{word, nact, g.nblk, !FUSED && a.staged, 0u, false};
     if (g.bid < nact) ok = op_chip<KIND, C64>(a, g, sh, X, gate, step, smem);
     else if (KIND != K_PERM) gate_arrive(gate);
-  } else if constexpr (STAGED) {
-    Gate gate{word, g.nblk, g.nblk, 0u};
+    off = gate.off;
+  } else if (X.bad || !FUSED) {
+    if (tid == 0) sh.R = OpResult{};
+    if (g.bid == 0 && tid == 0) op_refuse(a, C64);
+    // block 0 closes the op below: the others must have read its descriptors
+    Gate gate{word, 1, g.nblk, 0, 0u, false};
+    gate_arrive(gate);
+    if (g.bid == 0) ok = gate_wait(gate, a.ctrl);
+  } else if constexpr (FUSED) {
+    Gate gate{word, g.nblk, g.nblk, 0, 0u, false};
     ok = op_staged<KIND, C64>(a, g, sh, X, gate, smem);
   }
   pdl_trigger();
-  // every block knows the result; the last one out only resets the barrier
-  if (g.bid == 0 && ok) op_close(a, KIND, P_GATHER, P_GATHER, sh.R, n);
-  if (g.nblk > 1) op_exit(a.ctrl, g.nblk, !ok);
+  if (g.bid == 0 && !off) {
+    if (!FUSED && a.staged && tid == 0) {  // for the launches that follow
+      stage_of(a)->state = ST_OVER;
+      result_of(a)->failed = kOver;
+    }
+    // every block knows the result; the last one out only resets the barrier
+    if (ok) op_close(a, KIND, P_GATHER, P_GATHER, sh.R, n);
+  }
+  if (g.nblk > 1 && op_exit(a.ctrl, g.nblk, !ok && !off) == 3) {
+    // called off: the staged launches do the op
+    staged_zero(a, Grp{0, 1}, X.ntiles);
+    if (tid == 0) stage_of(a)->state = ST_OK;
+  }
 }
 
-// The chip route.
+// The staged route's later passes, each a launch.
 template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads, 4) k_op(const __grid_constant__ OpArgs a) {
-  pdl_wait();
-  op_body<KIND, C64, false>(a, whole_grid());
-}
-
-// One op on each of many states: every state's block group runs op_body with
-// the state's own workspace and control block (and so its own barriers).
-template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const SegPlan* plan) {
-  __shared__ OpArgs sa;
-  pdl_wait();  // the plan is the kernel before's
-  const Grp g = seg_enter(ops, plan, &sa, nullptr);
-  op_body<KIND, C64, true>(sa, g);
-}
-
-// The staged route, a launch per pass.
-template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads) k_op_zero(const __grid_constant__ OpArgs a) {
-  pdl_wait();
-  const OpCtx X = op_ctx<KIND, C64>(a);
-  if (!X.bad) staged_zero(a, whole_grid(), X);
-  pdl_trigger();
-}
-template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads) k_op_prep(const __grid_constant__ OpArgs a) {
+__device__ __forceinline__ void op_prep(const OpArgs& a, const Grp& g) {
   __shared__ FindSh F;
   __shared__ OpStage St;
-  pdl_wait();
+  const int state = KIND == K_PERM ? ST_OK : __ldcg(&stage_of(a)->state);
   const OpCtx X = op_ctx<KIND, C64>(a);
-  if (KIND == K_PERM && blockIdx.x == 0 && threadIdx.x < kOpCounters)
-    reinterpret_cast<unsigned long long*>(a.ws.counters)[threadIdx.x] = 0ULL;
-  if (!X.bad) staged_prep<KIND, C64>(a, whole_grid(), X);
-  else if (blockIdx.x == 0 && threadIdx.x == 0) op_refuse(a, C64);
+  if (KIND == K_PERM) {  // a reorder's first launch
+    if (g.bid == 0 && threadIdx.x < kOpCounters)
+      reinterpret_cast<unsigned long long*>(a.ws.counters)[threadIdx.x] = 0ULL;
+    if (X.bad && g.bid == 0 && threadIdx.x == 0) op_refuse(a, C64);
+    if (!X.bad) staged_prep<KIND, C64>(a, g, X);
+    pdl_trigger();
+    return;
+  }
+  if (state != ST_OK) return;
+  staged_prep<KIND, C64>(a, g, X);
   pdl_trigger();
-  if (KIND == K_PERM) return;
-  if (!op_exit(a.ctrl, gridDim.x, false)) return;
-  const Bracket B = X.bad ? Bracket{0ULL, 0ULL, 0, 0} : staged_bracket(a, X, F);
+  if (!op_exit(a.ctrl, g.nblk, false)) return;
+  const Bracket B = staged_bracket(a, X, F);
   if (threadIdx.x == 0) {
     St = OpStage{};
     St.B = B;
@@ -1844,55 +1887,53 @@ __global__ void __launch_bounds__(kThreads) k_op_prep(const __grid_constant__ Op
   store_words(a, kStageAt, St);
 }
 template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads, 4) k_op_eval(const __grid_constant__ OpArgs a) {
+__device__ __forceinline__ void op_eval(const OpArgs& a, const Grp& g) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ OpSh sh;
   if (threadIdx.x == 0) mbar_init(&sh.bar, 1);
-  pdl_wait();
   const OpCtx X = op_ctx<KIND, C64>(a);
   unsigned phase = 0;
   bool ok = true;
-  if (KIND == K_PERM) {
+  if constexpr (KIND == K_PERM) {
     __syncthreads();
     if (threadIdx.x == 0) sh.R = OpResult{};
     if (!X.bad) ok = staged_perm<C64>(a, sh, X, &phase, smem);
     pdl_trigger();
-    if (op_exit(a.ctrl, gridDim.x, !ok) == 1) op_close(a, KIND, P_HIST, P_HIST, sh.R, X.S.n);
-    return;
-  }
-  load_words(a, kStageAt, sh.St);
-  __syncthreads();
-  if (X.bad) return;
-  const Bracket B = sh.St.B;
-  ok = staged_eval<KIND, C64>(a, sh, X, B, &phase, smem);
-  pdl_trigger();
-  const int last = op_exit(a.ctrl, gridDim.x, !ok);
-  if (!last) return;
-  if (last == 1) {
-    staged_plan(a, sh, X, B);
+    if (op_exit(a.ctrl, g.nblk, !ok) == 1) op_close(a, KIND, P_HIST, P_HIST, sh.R, X.S.n);
   } else {
-    if (threadIdx.x == 0) sh.St.state = 2;
+    load_words(a, kStageAt, sh.St);
     __syncthreads();
+    if (sh.St.state != ST_OK) return;
+    const Bracket B = sh.St.B;
+    ok = staged_eval<KIND, C64>(a, sh, X, B, &phase, smem);
+    pdl_trigger();
+    const int last = op_exit(a.ctrl, g.nblk, !ok);
+    if (!last) return;
+    if (last == 1) {
+      staged_plan(a, sh, X, B);
+    } else {
+      if (threadIdx.x == 0) sh.St.state = ST_GAVE_UP;
+      __syncthreads();
+    }
+    store_words(a, kStageAt, sh.St);
   }
-  store_words(a, kStageAt, sh.St);
 }
 template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads, 4) k_op_settle(const __grid_constant__ OpArgs a) {
+__device__ __forceinline__ void op_settle(const OpArgs& a, const Grp& g) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ OpSh sh;
   if (threadIdx.x == 0) mbar_init(&sh.bar, 1);
-  pdl_wait();
   const OpCtx X = op_ctx<KIND, C64>(a);
-  if (X.bad) return;
   if (threadIdx.x == 0) op_preload(a, sh);
   load_words(a, kStageAt, sh.St);
   out_order_par(a.in, KIND, a.q, a.gb, sh.qat);
   __syncthreads();
-  Gate gate{reinterpret_cast<unsigned*>(&a.ctrl->sync_counter), (int)gridDim.x, (int)gridDim.x, 0u};
+  if (sh.St.state == ST_OVER) return;
+  Gate gate{reinterpret_cast<unsigned*>(&a.ctrl->sync_counter), g.nblk, g.nblk, 0, 0u, false};
   unsigned phase = 0;
-  const bool ok = sh.St.state != 2 && staged_settle<KIND, C64>(a, whole_grid(), sh, X, gate, &phase, smem);
+  const bool ok = sh.St.state != ST_GAVE_UP && staged_settle<KIND, C64>(a, g, sh, X, gate, &phase, smem);
   pdl_trigger();
-  const int last = op_exit(a.ctrl, gridDim.x, !ok);
+  const int last = op_exit(a.ctrl, g.nblk, !ok);
   if (!last) return;
   if (last == 1) {
     staged_final<KIND>(a, sh, X, smem);
@@ -1906,9 +1947,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_settle(const __grid_constant
   store_words(a, kResultAt, sh.R);
 }
 template <int KIND, bool C64>
-__global__ void __launch_bounds__(kThreads, 4) k_op_write(const __grid_constant__ OpArgs a) {
+__device__ __forceinline__ void op_write(const OpArgs& a, const Grp& g) {
   __shared__ OpSh sh;
-  pdl_wait();
   const OpCtx X = op_ctx<KIND, C64>(a);
   if (threadIdx.x == 0) op_preload(a, sh);
   if (X.bad) {
@@ -1917,18 +1957,56 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_write(const __grid_constant_
     load_words(a, kResultAt, sh.R);
   }
   __syncthreads();
-  if (!X.bad && !sh.R.failed) staged_write<KIND, C64>(a, whole_grid(), sh, X);
+  if (!X.bad && !sh.R.failed) staged_write<KIND, C64>(a, g, sh, X);
   pdl_trigger();
-  if (op_exit(a.ctrl, gridDim.x, sh.R.failed != 0) == 1) op_close(a, KIND, P_HIST, P_WRITE, sh.R, X.S.n);
+  if (sh.R.failed == kOver) return;
+  if (op_exit(a.ctrl, g.nblk, sh.R.failed != 0) == 1) op_close(a, KIND, P_HIST, P_WRITE, sh.R, X.S.n);
+}
+
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_first<KIND, C64, false>(a, whole_grid());
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads) k_op_prep(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_prep<KIND, C64>(a, whole_grid());
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_eval(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_eval<KIND, C64>(a, whole_grid());
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_settle(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_settle<KIND, C64>(a, whole_grid());
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_write(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_write<KIND, C64>(a, whole_grid());
+}
+
+// One op on each of many states: every state's block group runs both routes
+// with the state's own workspace and control block (and so its own barriers).
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const SegPlan* plan) {
+  __shared__ OpArgs sa;
+  pdl_wait();  // the plan is the kernel before's
+  const Grp g = seg_enter(ops, plan, &sa, nullptr);
+  op_first<KIND, C64, true>(sa, g);
 }
 
 // ---------------------------------------------------------------------------
 // launch
 // ---------------------------------------------------------------------------
-// op_exit counts the blocks in 11 bits; a chip op keeps a count per block in
+// op_exit counts the blocks in 10 bits; a chip op keeps a count per block in
 // the smallest workspace's partition records (3 x 6 words per set)
-constexpr int kOpMaxBlocks = 1024;
-static_assert(kOpMaxBlocks < 2047 && kOpMaxBlocks <= kMaxSets * 3 * 6, "block counts");
+constexpr int kOpMaxBlocks = 1023;
+static_assert(kOpMaxBlocks <= (int)kExitMask && kOpMaxBlocks <= kMaxSets * 3 * 6, "block counts");
+
 constexpr size_t kFusedSmem = kTileSmem > kChipSmem ? kTileSmem : kChipSmem;
 
 // Resident grid of a kernel of kThreads threads (at most kOpMaxBlocks).
@@ -1947,47 +2025,51 @@ static cudaError_t op_grid(PerDevice& cache, K kern, size_t smem, int* grid) {
   });
 }
 
+// The grids of a kind's launches.
+struct OpGrids {
+  int first, prep, eval, settle, write;
+};
 template <int KIND, bool C64>
-static cudaError_t launch_staged(const OpArgs& a, cudaStream_t s) {
-  static PerDevice ge, gs, gw, gp;
-  int eval = 0, settle = 0, write = 0, prep = 0;
-  cudaError_t e = op_grid(ge, k_op_eval<KIND, C64>, kTileSmem, &eval);
-  if (e == cudaSuccess) e = op_grid(gp, k_op_prep<KIND, C64>, 0, &prep);
-  if (e != cudaSuccess) return e;
+static cudaError_t op_grids(OpGrids* g) {
+  static PerDevice cf, cp, ce, cs, cw;
+  cudaError_t e = op_grid(cf, k_op<KIND, C64>, kChipSmem, &g->first);
+  if (e == cudaSuccess) e = op_grid(cp, k_op_prep<KIND, C64>, 0, &g->prep);
+  if (e == cudaSuccess) e = op_grid(ce, k_op_eval<KIND, C64>, kTileSmem, &g->eval);
   if constexpr (KIND != K_PERM) {
-    if ((e = op_grid(gs, k_op_settle<KIND, C64>, kTileSmem, &settle)) != cudaSuccess) return e;
-    if ((e = op_grid(gw, k_op_write<KIND, C64>, 0, &write)) != cudaSuccess) return e;
-    KLAUNCH(S_ZERO, s, e = launch_pdl(k_op_zero<KIND, C64>, dim3(64), dim3(kThreads), 0, s, a));
-    if (e != cudaSuccess) return e;
-  }
-  KLAUNCH(S_PARTITION, s, e = launch_pdl(k_op_prep<KIND, C64>, dim3(prep), dim3(kThreads), 0, s, a));
-  if (e != cudaSuccess) return e;
-  KLAUNCH(KIND * 5 + P_HIST, s, e = launch_pdl(k_op_eval<KIND, C64>, dim3(eval), dim3(kThreads), kTileSmem, s, a));
-  if (e != cudaSuccess) return e;
-  if constexpr (KIND != K_PERM) {
-    KLAUNCH(KIND * 5 + P_HIST2, s,
-            e = launch_coop(k_op_settle<KIND, C64>, dim3(settle), dim3(kThreads), kTileSmem, s, a));
-    if (e != cudaSuccess) return e;
-    KLAUNCH(KIND * 5 + P_WRITE, s, e = launch_pdl(k_op_write<KIND, C64>, dim3(write), dim3(kThreads), 0, s, a));
+    if (e == cudaSuccess) e = op_grid(cs, k_op_settle<KIND, C64>, kTileSmem, &g->settle);
+    if (e == cudaSuccess) e = op_grid(cw, k_op_write<KIND, C64>, 0, &g->write);
   }
   return e;
 }
 
 template <int KIND, bool C64>
-static cudaError_t launch_op(const OpArgs& a, cudaStream_t s) {
-  static PerDevice cache;
-  int grid = 0;
-  cudaError_t e = op_grid(cache, k_op<KIND, C64>, kChipSmem, &grid);
+static cudaError_t launch_op(OpArgs a, cudaStream_t s) {
+  OpGrids g{};
+  cudaError_t e = op_grids<KIND, C64>(&g);
   if (e != cudaSuccess) return e;
   // the workspace bounds the entries (the kernels refuse more)
   const long long bound = a.ws.max_n / slots_per_entry(KIND);
-  if (bound > (long long)grid * kChipStep) return launch_staged<KIND, C64>(a, s);
+  a.staged = bound > (long long)g.first * kChipStep;
   const long long want = bound <= kChipStep ? 1 : (bound + kChipMin - 1) / kChipMin;
-  if (want < grid) grid = (int)want;
-  if (grid == 1)  // no barrier
-    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op<KIND, C64>, dim3(1), dim3(kThreads), kChipSmem, s, a));
-  else
-    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op<KIND, C64>, dim3(grid), dim3(kThreads), kChipSmem, s, a));
+  if (a.staged) g.first = kFirstBlocks;
+  else if (want < g.first) g.first = (int)want;
+  if (a.staged || g.first == 1) {  // no barrier, or one that may be called off
+    if (KIND != K_PERM || !a.staged)  // (a staged reorder has nothing to clear)
+      KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
+  } else {
+    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
+  }
+  if (e != cudaSuccess || !a.staged) return e;
+  KLAUNCH(S_PARTITION, s, e = launch_pdl(k_op_prep<KIND, C64>, dim3(g.prep), dim3(kThreads), 0, s, a));
+  if (e != cudaSuccess) return e;
+  KLAUNCH(KIND * 5 + P_HIST, s, e = launch_pdl(k_op_eval<KIND, C64>, dim3(g.eval), dim3(kThreads), kTileSmem, s, a));
+  if constexpr (KIND != K_PERM) {
+    if (e != cudaSuccess) return e;
+    KLAUNCH(KIND * 5 + P_HIST2, s,
+            e = launch_coop(k_op_settle<KIND, C64>, dim3(g.settle), dim3(kThreads), kTileSmem, s, a));
+    if (e != cudaSuccess) return e;
+    KLAUNCH(KIND * 5 + P_WRITE, s, e = launch_pdl(k_op_write<KIND, C64>, dim3(g.write), dim3(kThreads), 0, s, a));
+  }
   return e;
 }
 
