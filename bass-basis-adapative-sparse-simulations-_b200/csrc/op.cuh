@@ -59,8 +59,10 @@ constexpr int kRegion = 32 * kPerThread;         // Z positions of a warp's regi
 constexpr int kRegions = kThreads / 32;          // regions of a tile
 // Blocks of a staged op's first launch: they do the whole op for a state of up
 // to kFirstBlocks x kChipStep = 32,512 entries under a larger bound.  One per SM
-// (148) would take states of 75,000 entries, but costs every op at 2^22 entries
-// 3 us (202 instead of 199), and at 65,536 entries the staged route is as fast.
+// (148) would take states of 75,000 entries, but costs a gate at 2^22 entries
+// 3 us (202 instead of 199), and at 65,536 entries its staged route is as fast.
+// A truncation takes one per SM: staged it is slower there (65,536 entries: 51 us
+// instead of 37), and at 2^22 no difference shows.
 constexpr int kFirstBlocks = 64;
 // |a|^2 bins of the sample: 128 per power of two over [2^-64, 1)
 constexpr int kSampleBase = (1023 - 64) << 7;
@@ -2051,7 +2053,7 @@ static cudaError_t launch_op(OpArgs a, cudaStream_t s) {
   const long long bound = a.ws.max_n / slots_per_entry(KIND);
   a.staged = bound > (long long)g.first * kChipStep;
   const long long want = bound <= kChipStep ? 1 : (bound + kChipMin - 1) / kChipMin;
-  if (a.staged) g.first = kFirstBlocks;
+  if (a.staged) g.first = KIND == K_IDENT ? device().sms : kFirstBlocks;
   else if (want < g.first) g.first = (int)want;
   if (a.staged || g.first == 1) {  // no barrier, or one that may be called off
     if (KIND != K_PERM || !a.staged)  // (a staged reorder has nothing to clear)

@@ -11,6 +11,7 @@ pytestmark = pytest.mark.gpu
 
 CHIP, EVAL, WRITE = 2, 0, 3          # passes of an op kind's profile slots
 FIRST = 64 * 508                     # entries the first launch's blocks hold
+FIRST_TOPK = 148 * 508               # ... of a truncation: a block per SM
 N = 36
 
 
@@ -66,7 +67,7 @@ def _want(orc, x, a, op, k):
 
 
 @pytest.mark.parametrize("op,kind", [("gate1", 0), ("rot", 1), ("gate2", 2), ("topk", 4)])
-@pytest.mark.parametrize("n", [3, 508, 509, FIRST, FIRST + 1])
+@pytest.mark.parametrize("n", [3, 508, 509, FIRST, FIRST + 1, FIRST_TOPK, FIRST_TOPK + 1])
 def test_small_state_under_a_large_bound(pkg, orc, n, op, kind):
     from bass_b200 import _native as nat
     k = max(1, (2 * n) // 3)
@@ -83,7 +84,7 @@ def test_small_state_under_a_large_bound(pkg, orc, n, op, kind):
     wx, wa = _want(orc, x, a, op, k)
     assert np.array_equal(st.x, wx) and np.array_equal(st.alpha, wa)
     want = np.zeros(5, np.int64)
-    want[CHIP if n <= FIRST else EVAL] = n
+    want[CHIP if n <= (FIRST_TOPK if op == "topk" else FIRST) else EVAL] = n
     assert c["prof_in"][5 * kind:5 * kind + 5].tolist() == want.tolist()
 
 
