@@ -338,9 +338,34 @@ __device__ __forceinline__ void tile_merge(const TileSeg& T, const uint64_t* sK,
   __syncthreads();
 }
 
+// Z order of a tile when the target bit is already in its place (t == GB): the
+// order of the keys, in which the segments were loaded.
+template <int PT, int GB>
+__device__ __forceinline__ void tile_in_order(const TileSeg& T, const uint64_t* sK, uint16_t* sP) {
+  const int E = (int)T.off[5];
+  const int o1 = (int)T.off[1], o2 = (int)T.off[2], o3 = (int)T.off[3], o4 = (int)T.off[4];
+  auto place = [&](int e) { return e + T.gap[(e >= o1) + (e >= o2) + (e >= o3) + (e >= o4)]; };
+#pragma unroll
+  for (int k = 0; k < PT; ++k) {
+    const int p = k * kThreads + (int)threadIdx.x;
+    if (p >= E) break;
+    const int q = place(p);
+    const uint64_t key = sK[q], group = key >> (GB + 1);
+    const bool same = p > 0 && (sK[place(p - 1)] >> (GB + 1)) == group;
+    const bool next = p + 1 < E && (sK[place(p + 1)] >> (GB + 1)) == group;
+    const unsigned local = (unsigned)key & ((2u << GB) - 1u);
+    sP[p] = (uint16_t)((unsigned)q | (local << kPlaceLocal) | (next ? kPlaceNext : 0u) | (same ? 0u : kPlaceStart));
+  }
+  __syncthreads();
+}
+
 template <int PT, int GB>
 __device__ __forceinline__ void tile_zorder(const TileSeg& T, const uint64_t* sK, uint16_t* sP, int* sWarp, int t) {
   const int E = (int)T.off[5];
+  if (t == GB) {
+    tile_in_order<PT, GB>(T, sK, sP);
+    return;
+  }
   if (T.off[2] == E) {  // two segments: the runs themselves
     tile_merge<PT, GB, false>(T, sK, sP, (int)T.off[1], t);
     return;
