@@ -98,6 +98,9 @@ class StatePool:
         self.kron = [dict() for _ in range(S)]
         self.pcur, self.ptmp, self.ptmp2, self.pctrl, self.pws, self.wsb, self.prho = (
             np.zeros(S, np.uint64) for _ in range(7))
+        # the workspace sizes that bound ops of one, two and four children per
+        # entry: small states then need no staged launches
+        self.wsb_for = {s: np.zeros(S, np.uint64) for s in (1, 2, 4)}
         self.nq = np.zeros(S, np.int32)
         self.kk = np.zeros(S, np.int64)
         self.pos = np.zeros(S, np.int64)
@@ -148,6 +151,8 @@ class StatePool:
         ptr = nat._ptr
         self.pcur[c], self.ptmp[c], self.ptmp2[c] = ptr(st._cur.desc), ptr(st._tmp.desc), ptr(st._tmp2.desc)
         self.pctrl[c], self.pws[c], self.wsb[c], self.prho[c] = ptr(eng.ctrl), ptr(eng.ws), eng.ws_bytes, ptr(eng.rho)
+        for slots, b in self.wsb_for.items():
+            b[c] = eng.ws_for(cap, slots)
         self.nq[c], self.kk[c] = N, k
         self.pos[c], self.length[c] = 0, len(circuit)
         self.pr_last_opt[c] = 0.0
@@ -175,15 +180,16 @@ class StatePool:
         return st
 
     # ---- plumbing ------------------------------------------------------------------------
-    def _ops(self, idx):
-        """bass_seg_op rows for the slots idx (an int array)."""
+    def _ops(self, idx, slots=None):
+        """bass_seg_op rows for the slots idx (an int array); slots: the most
+        children per entry of the op, if it has any."""
         o = np.zeros(len(idx), dtype=nat.SEG_OP_DTYPE)
         o["in"] = self.pcur[idx]
         o["tmp"] = self.ptmp[idx]
         o["out"] = self.ptmp2[idx]
         o["ctrl"] = self.pctrl[idx]
         o["ws"] = self.pws[idx]
-        o["ws_bytes"] = self.wsb[idx]
+        o["ws_bytes"] = (self.wsb if slots is None else self.wsb_for[slots])[idx]
         o["rho"] = self.prho[idx]
         o["num_qubits"] = self.nq[idx]
         o["k_cond"] = -1
@@ -240,7 +246,7 @@ class StatePool:
         o["mark_active"] = 1
 
     def _gate1(self, idx, q, G):
-        o = self._ops(idx)
+        o = self._ops(idx, 2)
         o["q1"] = q
         o["G"][:, :8] = np.ascontiguousarray(G).view(np.float64).reshape(len(idx), 8)
         self._fused(o, idx)
@@ -248,7 +254,7 @@ class StatePool:
         self._swap(self.pcur, self.ptmp2, idx)   # the op wrote its "out" descriptor
 
     def _gate2(self, idx, qa, qb, G):
-        o = self._ops(idx)
+        o = self._ops(idx, 4)
         o["q1"] = qa
         o["q2"] = qb
         o["G"][:, :32] = np.ascontiguousarray(G).view(np.float64).reshape(len(idx), 32)
@@ -365,7 +371,7 @@ class StatePool:
                 if not len(rr):
                     continue
                 idx = active[rr]
-                oj = self._ops(idx)
+                oj = self._ops(idx, 2)
                 oj["q1"] = jq
                 Uh = np.ascontiguousarray(np.conj(np.swapaxes(Vs[rr, jq], 1, 2)))
                 oj["G"][:, :8] = Uh.view(np.float64).reshape(len(rr), 8)
@@ -388,7 +394,7 @@ class StatePool:
             active = active[improved]
             if not len(active):
                 break
-        o = self._ops(T)
+        o = self._ops(T, 1)
         o["k_cond"] = self.kk[T]
         o["k_keep"] = self.kk[T]
         self._call("bass_topk_batch", o)                 # _truncate_state

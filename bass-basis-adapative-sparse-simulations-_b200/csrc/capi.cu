@@ -610,8 +610,10 @@ int bass_gate_1q_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t bat
     load_G(A[i], o.G, 4);
   }
   if (!same_type(A)) return BASS_ERR_ARG;
-  cudaError_t e = upload(bv.ops_a, A, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE1, bv.ops_a, n, A[0].c64, bv.plan, s);
+  int staged = 0;
+  cudaError_t e = seg_stages(K_GATE1, A.data(), n, 2, &staged);
+  if (e == cudaSuccess) e = upload(bv.ops_a, A, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE1, bv.ops_a, n, A[0].c64, staged, bv.plan, s);
   return status_of(e);
 }
 
@@ -637,10 +639,15 @@ int bass_gate_2q_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t bat
     load_G(B[i], o.G, 16);
   }
   if (!same_type(A)) return BASS_ERR_ARG;
-  cudaError_t e = upload(bv.ops_a, A, s);
+  // (the gate takes a quarter of the entries that the workspace holds, and so
+  // the reorder before it)
+  int staged_a = 0, staged_b = 0;
+  cudaError_t e = seg_stages(K_PERM, A.data(), n, 4, &staged_a);
+  if (e == cudaSuccess) e = seg_stages(K_GATE2, B.data(), n, 4, &staged_b);
+  if (e == cudaSuccess) e = upload(bv.ops_a, A, s);
   if (e == cudaSuccess) e = upload(bv.ops_b, B, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_PERM, bv.ops_a, n, A[0].c64, bv.plan, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE2, bv.ops_b, n, A[0].c64, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_PERM, bv.ops_a, n, A[0].c64, staged_a, bv.plan, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_GATE2, bv.ops_b, n, A[0].c64, staged_b, bv.plan, s);
   return status_of(e);
 }
 
@@ -668,8 +675,10 @@ int bass_topk_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t batch_
     if (!seg_common(o, &A[i]) || !o.out || o.out == o.in) return BASS_ERR_ARG;
   }
   if (!same_type(A)) return BASS_ERR_ARG;
-  cudaError_t e = upload(bv.ops_a, A, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_IDENT, bv.ops_a, n, A[0].c64, bv.plan, s);
+  int staged = 0;
+  cudaError_t e = seg_stages(K_IDENT, A.data(), n, 1, &staged);
+  if (e == cudaSuccess) e = upload(bv.ops_a, A, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_IDENT, bv.ops_a, n, A[0].c64, staged, bv.plan, s);
   return status_of(e);
 }
 
@@ -689,8 +698,10 @@ int bass_rotate_step_batch(const bass_seg_op* ops, int n, void* batch_ws, size_t
     load_G(A[i], o.G, 4);
   }
   if (!same_type(A)) return BASS_ERR_ARG;
-  cudaError_t e = upload(bv.ops_a, A, s);
-  if (e == cudaSuccess) e = run_merge_op_seg(K_ROT1, bv.ops_a, n, A[0].c64, bv.plan, s);
+  int staged = 0;
+  cudaError_t e = seg_stages(K_ROT1, A.data(), n, 2, &staged);
+  if (e == cudaSuccess) e = upload(bv.ops_a, A, s);
+  if (e == cudaSuccess) e = run_merge_op_seg(K_ROT1, bv.ops_a, n, A[0].c64, staged, bv.plan, s);
   return status_of(e);
 }
 

@@ -33,6 +33,7 @@ struct OpArgs {
   int prof;       // count entries into ctrl->prof_in / prof_out
   int fin_mode;   // 0 gate / truncation, 1 rotation step
   int staged;     // launches of the staged route follow the first one
+  int seg;        // a segmented op
   int commit;     // rotation step: the op also commits (swaps in an accepted candidate)
   int j;          // rotation step: the rotated qubit
   long long k_cond, k_keep;
@@ -51,6 +52,10 @@ struct SegPlan {
   int kind;
   long long wp[kMaxSeg + 1];  // exclusive prefix of the states' work weights
 };
+
+// Added to a state's entries in an op's work weight: a state gets blocks in
+// proportion, beside the one that each has.
+constexpr int kSegPad = 252;
 
 enum Slot {
   S_PARTITION = 30, S_ZERO = 31, S_REDUCE = 35,
@@ -154,7 +159,10 @@ cudaError_t run_commit(bass_state* cur, bass_state* tmp, bass_ctrl* ctrl, const 
 
 // merge.cu, segmented: ops_dev holds nseg OpArgs (all of one amplitude type),
 // plan_dev is scratch for the block groups
-cudaError_t run_merge_op_seg(int kind, const OpArgs* ops_dev, int nseg, int c64, SegPlan* plan_dev, cudaStream_t s);
+cudaError_t run_merge_op_seg(int kind, const OpArgs* ops_dev, int nseg, int c64, int staged, SegPlan* plan_dev,
+                             cudaStream_t s);
+// sets the ops' launches (OpArgs::staged) before they are copied to the device
+cudaError_t seg_stages(int kind, OpArgs* ops, int nseg, int slots, int* staged);
 cudaError_t run_seg_plan(const OpArgs* ops_dev, int nseg, int kind, SegPlan* plan_dev, cudaStream_t s);
 cudaError_t run_rdm_seg(const OpArgs* ops_dev, int nseg, int max_nq, int c64, SegPlan* plan_dev, cudaStream_t s);
 // the most segments one segmented launch takes on the current device

@@ -762,12 +762,12 @@ cudaError_t run_rdm_prepared(const bass_state* st, int nq, double* rho, bass_ctr
 // segmented launches: one op on each of many states per launch
 // ---------------------------------------------------------------------------
 // The block groups of an op: work weight of state s = its input entries plus
-// one tile (times its qubits for an RDM).  One block.
+// kSegPad (an RDM's: plus one tile, times its qubits).  One block.
 __global__ void k_seg_plan(const OpArgs* ops, int nseg, int kind, SegPlan* plan) {
   __shared__ long long sW[kMaxSeg];
   for (int s = threadIdx.x; s < nseg; s += blockDim.x) {
     const long long n = ops[s].in->nnz;
-    sW[s] = (n + kStep) * (kind == K_RDM ? (long long)ops[s].nsets : 1LL);
+    sW[s] = kind == K_RDM ? (n + kStep) * (long long)ops[s].nsets : n + kSegPad;
   }
   __syncthreads();
   if (threadIdx.x == 0) {

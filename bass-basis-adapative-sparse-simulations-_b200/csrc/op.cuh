@@ -53,8 +53,8 @@ constexpr int kChipPad = kChipTile + 8;
 constexpr int kChipBins = 2048;                  // digits of the chip search: 11 bits (the first: the exponent)
 constexpr int kChipLate = 32;                    // undecided children it stops at (one per lane of a warp)
 constexpr int kSelMax = 256;                     // boundary children settled by ranking (one per thread)
-constexpr int kSamples = 16384;                  // sampled entries of the bracket
-constexpr int kSampleMargin = 512;               // 4 sqrt(kSamples): ranks around the estimate
+constexpr int kSamples = 16384;                  // sampled entries of the bracket, at most
+constexpr int kSampleRounds = 2;                 // ... per eight lanes of a group's blocks
 constexpr int kRegion = 32 * kPerThread;         // Z positions of a warp's region of a tile
 constexpr int kRegions = kThreads / 32;          // regions of a tile
 // Blocks of a staged op's first launch: they do the whole op for a state of up
@@ -1095,6 +1095,15 @@ __device__ __forceinline__ void sample_entry(const OpArgs& a, const OpCtx& X, lo
   }
 }
 
+// Sampled entries: no more than two rounds of the group's eights of lanes.  A
+// small group of a segmented op spends longer on a full sample's chains of loads
+// than a wider bracket costs (64 states of 32,768 entries: 204 us per gate with
+// two rounds, 208 with four, 224 with eight, summed over the launches).
+__device__ __forceinline__ long long sample_count(long long n, int nblk) {
+  const long long room = (long long)nblk * (kThreads / 8) * kSampleRounds;
+  const long long s = room < kSamples ? room : kSamples;
+  return n < s ? n : s;
+}
 __device__ __forceinline__ bool is_bracketed(const OpArgs& a, const OpCtx& X) { return X.may_trunc && a.k_keep > 0; }
 
 // Clears the counters, both histograms and the tiles' counts.
@@ -1124,7 +1133,7 @@ __device__ __forceinline__ void staged_prep(const OpArgs& a, const Grp& g, const
     }
   }
   if (KIND != K_PERM && is_bracketed(a, X)) {
-    const long long S = n < kSamples ? n : kSamples;
+    const long long S = sample_count(n, g.nblk);
     for (long long s = (gthreads - 1 - gtid) >> 3; s < S; s += gthreads >> 3) {
       // one entry of each of S equal ranges, at a hashed place in it
       const long long lo = s * n / S, hi = (s + 1) * n / S;
@@ -1134,15 +1143,15 @@ __device__ __forceinline__ void staged_prep(const OpArgs& a, const Grp& g, const
 }
 
 // Block-wide: the bracket, from the sample's histogram (every thread gets it).
-__device__ __forceinline__ Bracket staged_bracket(const OpArgs& a, const OpCtx& X, FindSh& F) {
+__device__ __forceinline__ Bracket staged_bracket(const OpArgs& a, const Grp& g, const OpCtx& X, FindSh& F) {
   Bracket B{0ULL, 0ULL, 0, 0};  // nothing is dropped: every child certain
   if (!is_bracketed(a, X)) return B;
-  const long long n = X.S.n, S = n < kSamples ? n : kSamples;
+  const long long n = X.S.n, S = sample_count(n, g.nblk);
   // ranks k S / n -+ the margin of the sampled children
   unsigned long long s, x;
   top_scan<true, kHistBins>(a.ws.hist1, F, &s, &x);
   const long long r = (long long)(((unsigned __int128)a.k_keep * (unsigned long long)S) / (unsigned long long)n);
-  const long long margin = S < n ? kSampleMargin : 0;
+  const long long margin = S < n ? (long long)(4.0f * sqrtf((float)S)) : 0;  // four deviations of a rank
   const long long rh = r - margin, rl = r + margin + (S < n ? 1 : 0);
   B.hi = ~0ULL;
   if (rh >= 1) {
@@ -1764,46 +1773,15 @@ __device__ __forceinline__ void op_close(const OpArgs& a, int kind, int pass_in,
   op_finalize(a, kind, R);
 }
 
-// The staged route as one kernel of barriers (segmented ops: a group's route
-// depends on its state).
-template <int KIND, bool C64>
-__device__ __forceinline__ bool op_staged(const OpArgs& a, const Grp& g, OpSh& sh, const OpCtx& X, Gate& gate,
-                                          unsigned char* smem) {
-  unsigned phase = 0;
-  staged_zero(a, g, X.ntiles);
-  if (!gate_sync(gate, a.ctrl)) return false;
-  staged_prep<KIND, C64>(a, g, X);
-  if (!gate_sync(gate, a.ctrl)) return false;
-  if constexpr (KIND == K_PERM) {
-    return staged_perm<C64>(a, sh, X, &phase, smem);
-  } else {
-    const Bracket B = staged_bracket(a, X, sh.F);
-    if (!staged_eval<KIND, C64>(a, sh, X, B, &phase, smem)) return false;
-    if (!gate_sync(gate, a.ctrl)) return false;
-    staged_plan(a, sh, X, B);
-    if (!staged_settle<KIND, C64>(a, g, sh, X, gate, &phase, smem)) return false;
-    if (!gate_sync(gate, a.ctrl)) return false;
-    if (g.bid == 0) {
-      staged_final<KIND>(a, sh, X, smem);
-      store_words(a, kResultAt, sh.R);
-    }
-    if (!gate_sync(gate, a.ctrl)) return false;
-    load_words(a, kResultAt, sh.R);
-    __syncthreads();
-    staged_write<KIND, C64>(a, g, sh, X);
-    return true;
-  }
-}
-
 // The first launch of an op: the whole op on the chip route if the group's
 // blocks can hold the state, otherwise (a.staged) the staged route's clearing.
 // The later launches of an op that is over return at once.
-template <int KIND, bool C64, bool FUSED>
+template <int KIND, bool C64>
 __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ OpSh sh;
   const int tid = threadIdx.x;
-  if (!FUSED && a.staged) {
+  if (a.staged) {
     // too large for the chip route and accepted: as little code as can be (its
     // lines come from DRAM after an op on a large state)
     const long long n = a.in->nnz, nt = KIND == K_IDENT ? plain_tiles(n) : merge_tiles(n);
@@ -1830,24 +1808,21 @@ __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
     // descriptors, which block 0 rewrites at the end), the ones with a tile
     // at the others
     const int nact = n > 0 ? (int)((n + step - 1) / step) : 1;
-    Gate gate{word, nact, g.nblk, !FUSED && a.staged, 0u, false};
+    Gate gate{word, nact, g.nblk, a.staged, 0u, false};
     if (g.bid < nact) ok = op_chip<KIND, C64>(a, g, sh, X, gate, step, smem);
     else if (KIND != K_PERM) gate_arrive(gate);
     off = gate.off;
-  } else if (X.bad || !FUSED) {
+  } else {
     if (tid == 0) sh.R = OpResult{};
     if (g.bid == 0 && tid == 0) op_refuse(a, C64);
     // block 0 closes the op below: the others must have read its descriptors
     Gate gate{word, 1, g.nblk, 0, 0u, false};
     gate_arrive(gate);
     if (g.bid == 0) ok = gate_wait(gate, a.ctrl);
-  } else if constexpr (FUSED) {
-    Gate gate{word, g.nblk, g.nblk, 0, 0u, false};
-    ok = op_staged<KIND, C64>(a, g, sh, X, gate, smem);
   }
   pdl_trigger();
   if (g.bid == 0 && !off) {
-    if (!FUSED && a.staged && tid == 0) {  // for the launches that follow
+    if (a.staged && tid == 0) {  // for the launches that follow
       stage_of(a)->state = ST_OVER;
       result_of(a)->failed = kOver;
     }
@@ -1866,9 +1841,11 @@ template <int KIND, bool C64>
 __device__ __forceinline__ void op_prep(const OpArgs& a, const Grp& g) {
   __shared__ FindSh F;
   __shared__ OpStage St;
-  const int state = KIND == K_PERM ? ST_OK : __ldcg(&stage_of(a)->state);
+  const bool first = KIND == K_PERM && !a.seg;  // a plain reorder has no launch before this one
+  const int state = first ? ST_OK : __ldcg(&stage_of(a)->state);
   const OpCtx X = op_ctx<KIND, C64>(a);
-  if (KIND == K_PERM) {  // a reorder's first launch
+  if (state != ST_OK) return;
+  if (KIND == K_PERM) {
     if (g.bid == 0 && threadIdx.x < kOpCounters)
       reinterpret_cast<unsigned long long*>(a.ws.counters)[threadIdx.x] = 0ULL;
     if (X.bad && g.bid == 0 && threadIdx.x == 0) op_refuse(a, C64);
@@ -1876,11 +1853,10 @@ __device__ __forceinline__ void op_prep(const OpArgs& a, const Grp& g) {
     pdl_trigger();
     return;
   }
-  if (state != ST_OK) return;
   staged_prep<KIND, C64>(a, g, X);
   pdl_trigger();
   if (!op_exit(a.ctrl, g.nblk, false)) return;
-  const Bracket B = staged_bracket(a, X, F);
+  const Bracket B = staged_bracket(a, g, X, F);
   if (threadIdx.x == 0) {
     St = OpStage{};
     St.B = B;
@@ -1897,6 +1873,7 @@ __device__ __forceinline__ void op_eval(const OpArgs& a, const Grp& g) {
   unsigned phase = 0;
   bool ok = true;
   if constexpr (KIND == K_PERM) {
+    if (a.seg && __ldcg(&stage_of(a)->state) != ST_OK) return;
     __syncthreads();
     if (threadIdx.x == 0) sh.R = OpResult{};
     if (!X.bad) ok = staged_perm<C64>(a, sh, X, &phase, smem);
@@ -1968,7 +1945,7 @@ __device__ __forceinline__ void op_write(const OpArgs& a, const Grp& g) {
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads, 4) k_op(const __grid_constant__ OpArgs a) {
   pdl_wait();
-  op_first<KIND, C64, false>(a, whole_grid());
+  op_first<KIND, C64>(a, whole_grid());
 }
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads) k_op_prep(const __grid_constant__ OpArgs a) {
@@ -1991,14 +1968,47 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_write(const __grid_constant_
   op_write<KIND, C64>(a, whole_grid());
 }
 
-// One op on each of many states: every state's block group runs both routes
+// One op on each of many states: every state's block group runs the same passes
 // with the state's own workspace and control block (and so its own barriers).
+// (As one kernel of both routes they spilled 700 to 2,300 bytes a thread and
+// waited at grid barriers between the passes: 64 states of 32,768 entries took
+// 431 us per 1-qubit gate.)
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const SegPlan* plan) {
   __shared__ OpArgs sa;
   pdl_wait();  // the plan is the kernel before's
   const Grp g = seg_enter(ops, plan, &sa, nullptr);
-  op_first<KIND, C64, true>(sa, g);
+  op_first<KIND, C64>(sa, g);
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads) k_op_prep_seg(const OpArgs* ops, const SegPlan* plan) {
+  __shared__ OpArgs sa;
+  pdl_wait();
+  const Grp g = seg_enter(ops, plan, &sa, nullptr);
+  op_prep<KIND, C64>(sa, g);
+}
+// (three blocks per SM: with the op's arguments in shared memory four spill; 148
+// states of 2048 entries 52 -> 40 us, 64 of 32,768 81 -> 75)
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 3) k_op_eval_seg(const OpArgs* ops, const SegPlan* plan) {
+  __shared__ OpArgs sa;
+  pdl_wait();
+  const Grp g = seg_enter(ops, plan, &sa, nullptr);
+  op_eval<KIND, C64>(sa, g);
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_settle_seg(const OpArgs* ops, const SegPlan* plan) {
+  __shared__ OpArgs sa;
+  pdl_wait();
+  const Grp g = seg_enter(ops, plan, &sa, nullptr);
+  op_settle<KIND, C64>(sa, g);
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_write_seg(const OpArgs* ops, const SegPlan* plan) {
+  __shared__ OpArgs sa;
+  pdl_wait();
+  const Grp g = seg_enter(ops, plan, &sa, nullptr);
+  op_write<KIND, C64>(sa, g);
 }
 
 // ---------------------------------------------------------------------------
@@ -2008,8 +2018,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const
 // the smallest workspace's partition records (3 x 6 words per set)
 constexpr int kOpMaxBlocks = 1023;
 static_assert(kOpMaxBlocks <= (int)kExitMask && kOpMaxBlocks <= kMaxSets * 3 * 6, "block counts");
-
-constexpr size_t kFusedSmem = kTileSmem > kChipSmem ? kTileSmem : kChipSmem;
 
 // Resident grid of a kernel of kThreads threads (at most kOpMaxBlocks).
 template <typename K>
@@ -2083,28 +2091,68 @@ cudaError_t merge_op(const OpArgs& a, cudaStream_t s) {
 // ---- segmented ------------------------------------------------------------------
 // Resident grid of the segmented op (at least one block per segment).
 template <int KIND, bool C64>
-cudaError_t seg_op_grid(int* grid) {
+static cudaError_t seg_op_grid(int* grid) {
   static PerDevice cache;
-  return op_grid(cache, k_op_seg<KIND, C64>, kFusedSmem, grid);
+  return op_grid(cache, k_op_seg<KIND, C64>, kChipSmem, grid);
 }
 
-template <int KIND, bool C64>
-static cudaError_t merge_op_seg(const OpArgs* ops, int nseg, SegPlan* plan, cudaStream_t s) {
+// Do the staged launches have to follow the first one?  Not if every state fits
+// its blocks however many entries it holds: with work weights n + kSegPad a
+// state gets more than (grid - nseg) (n + kSegPad) / W blocks, so W <= (grid -
+// nseg) kChipStep, which the workspaces' bounds show, is enough.  slots: children
+// per entry that the workspaces are sized for.
+template <int KIND>
+cudaError_t seg_stages_t(OpArgs* ops, int nseg, int slots, int* staged) {
   int grid = 0;
-  cudaError_t e = seg_op_grid<KIND, C64>(&grid);
+  const cudaError_t e = ops[0].c64 ? seg_op_grid<KIND, true>(&grid) : seg_op_grid<KIND, false>(&grid);
   if (e != cudaSuccess) return e;
-  int most = grid;  // the groups' barriers need every block resident
-  if (KIND != K_PERM && (e = seg_max_segments(&most)) != cudaSuccess) return e;
+  long long w = 0;
+  for (int i = 0; i < nseg; ++i) w += ops[i].ws.max_n / slots + kSegPad;
+  *staged = w > (long long)(grid - nseg) * kChipStep;
+  for (int i = 0; i < nseg; ++i) ops[i].staged = *staged, ops[i].seg = 1;
+  return cudaSuccess;
+}
+
+// The first launch is cooperative, since states that stay on chip share it.
+template <int KIND, bool C64>
+static cudaError_t merge_op_seg(const OpArgs* ops, int nseg, int staged, SegPlan* plan, cudaStream_t s) {
+  static PerDevice cp, ce, cs, cw;
+  OpGrids g{};
+  cudaError_t e = seg_op_grid<KIND, C64>(&g.first);
+  if (e == cudaSuccess) e = op_grid(cp, k_op_prep_seg<KIND, C64>, 0, &g.prep);
+  if (e == cudaSuccess) e = op_grid(ce, k_op_eval_seg<KIND, C64>, kTileSmem, &g.eval);
+  if constexpr (KIND != K_PERM) {
+    if (e == cudaSuccess) e = op_grid(cs, k_op_settle_seg<KIND, C64>, kTileSmem, &g.settle);
+    if (e == cudaSuccess) e = op_grid(cw, k_op_write_seg<KIND, C64>, 0, &g.write);
+  }
+  if (e != cudaSuccess) return e;
+  int most = g.first;  // the groups' barriers need every block resident
+  if (KIND != K_PERM && most > device().sms) most = device().sms;  // (seg_max_segments)
   if (nseg > most) return cudaErrorInvalidValue;
   if ((e = run_seg_plan(ops, nseg, KIND, plan, s)) != cudaSuccess) return e;
-  KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op_seg<KIND, C64>, dim3(grid), dim3(kThreads), kFusedSmem, s, ops,
-                                                (const SegPlan*)plan));
+  const SegPlan* p = plan;
+  KLAUNCH(KIND * 5 + P_GATHER, s,
+          e = launch_coop(k_op_seg<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, ops, p));
+  if (e != cudaSuccess || !staged) return e;
+  KLAUNCH(S_PARTITION, s, e = launch_pdl(k_op_prep_seg<KIND, C64>, dim3(g.prep), dim3(kThreads), 0, s, ops, p));
+  if (e != cudaSuccess) return e;
+  KLAUNCH(KIND * 5 + P_HIST, s,
+          e = launch_pdl(k_op_eval_seg<KIND, C64>, dim3(g.eval), dim3(kThreads), kTileSmem, s, ops, p));
+  if constexpr (KIND != K_PERM) {
+    if (e != cudaSuccess) return e;
+    KLAUNCH(KIND * 5 + P_HIST2, s,
+            e = launch_coop(k_op_settle_seg<KIND, C64>, dim3(g.settle), dim3(kThreads), kTileSmem, s, ops, p));
+    if (e != cudaSuccess) return e;
+    KLAUNCH(KIND * 5 + P_WRITE, s,
+            e = launch_pdl(k_op_write_seg<KIND, C64>, dim3(g.write), dim3(kThreads), 0, s, ops, p));
+  }
   return e;
 }
 
 template <int KIND>
-cudaError_t merge_op_seg_t(const OpArgs* ops, int nseg, int c64, SegPlan* plan, cudaStream_t s) {
-  return c64 ? merge_op_seg<KIND, true>(ops, nseg, plan, s) : merge_op_seg<KIND, false>(ops, nseg, plan, s);
+cudaError_t merge_op_seg_t(const OpArgs* ops, int nseg, int c64, int staged, SegPlan* plan, cudaStream_t s) {
+  return c64 ? merge_op_seg<KIND, true>(ops, nseg, staged, plan, s)
+             : merge_op_seg<KIND, false>(ops, nseg, staged, plan, s);
 }
 
 }  // namespace bass

@@ -3,5 +3,6 @@
 
 namespace bass {
 template cudaError_t merge_op<K_PERM>(const OpArgs&, cudaStream_t);
-template cudaError_t merge_op_seg_t<K_PERM>(const OpArgs*, int, int, SegPlan*, cudaStream_t);
+template cudaError_t merge_op_seg_t<K_PERM>(const OpArgs*, int, int, int, SegPlan*, cudaStream_t);
+template cudaError_t seg_stages_t<K_PERM>(OpArgs*, int, int, int*);
 }  // namespace bass
