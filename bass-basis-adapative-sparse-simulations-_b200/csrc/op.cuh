@@ -103,9 +103,8 @@ struct Gate {
   unsigned* word;
   int nact;         // blocks that take part
   int all;          // arrivals of the first barrier (every block of the launch may count there)
-  int may_off;      // the first barrier may be called off
   unsigned passed;  // barriers entered
-  bool off;         // it was
+  bool off;         // the launch was called off
 };
 
 // Block-wide: arrive (everything written before is visible to the blocks that
@@ -119,41 +118,42 @@ __device__ __forceinline__ void gate_arrive(Gate& b) {
   }
 }
 // Block-wide: wait until every block has arrived (bounded; false on give-up,
-// with BASS_ERR_WAIT recorded, and when the launch is called off).
+// with BASS_ERR_WAIT recorded).  OFF: the launch's first barrier, which may be
+// called off (false then too).
+template <bool OFF = false>
 __device__ __forceinline__ bool gate_wait(Gate& b, bass_ctrl* c) {
   __shared__ int sOk;  // 1 all arrived, 0 gave up, -1 called off
   if (b.nact > 1 || (b.passed == 1 && b.all > 1)) {
     if (threadIdx.x == 0) {
       const unsigned target = (unsigned)b.all + (b.passed - 1) * (unsigned)b.nact;
-      const bool may_off = b.may_off && b.passed == 1;
       long long lim = wait_limit(c);
-      if (may_off && lim > kOffSpins) lim = kOffSpins;
+      if (OFF && lim > kOffSpins) lim = kOffSpins;
       long long spins = 0;
       int ok = 1;
       for (;;) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(b.word) : "memory");
-        if (may_off && (v & kOffBit)) {
+        if (OFF && (v & kOffBit)) {
           ok = -1;
           break;
         }
         if ((v & kArriveMask) >= target) break;
         if (++spins > lim) {
-          if (!may_off) {
+          if (!OFF) {
             set_error(c, BASS_ERR_WAIT);
             ok = 0;
             break;
           }
           atomicCAS(b.word, v, v | kOffBit);  // (or the word has changed: look again)
-        } else {
-          __nanosleep(b.nact > 64 ? 100 : 20);  // (hundreds of pollers would hold up the arrivals)
+          continue;
         }
+        __nanosleep(b.nact > 64 ? 100 : 20);  // (hundreds of pollers would hold up the arrivals)
       }
       __threadfence();
       sOk = ok;
     }
     __syncthreads();
-    b.off = sOk < 0;
+    if (OFF) b.off = sOk < 0;
     return sOk > 0;
   }
   __syncthreads();
@@ -679,7 +679,7 @@ __device__ __forceinline__ void flush_sums(OpSh& sh, unsigned long long* cn, i12
 // ---- chip route -------------------------------------------------------------
 // Block b of nact holds tile b (step Z positions).  Returns false if a wait
 // gave up; otherwise sh.R is the op's result.
-template <int KIND, bool C64>
+template <int KIND, bool C64, bool OFF>
 __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh, const OpCtx& X, Gate& gate, int step,
                                         unsigned char* smem) {
   constexpr int NS = slots_per_entry(KIND);
@@ -777,7 +777,7 @@ __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh,
     nex += __popc(cm);
   }
   nex = (int)__reduce_add_sync(0xffffffffu, (unsigned)nex);
-  if (!gate_wait(gate, a.ctrl)) return false;
+  if (!gate_wait<OFF>(gate, a.ctrl)) return false;
   if (lane == 0 && nex) atomicAdd(cn + C_OUT, (unsigned long long)nex);
 
   // the threshold
@@ -1776,12 +1776,13 @@ __device__ __forceinline__ void op_close(const OpArgs& a, int kind, int pass_in,
 // The first launch of an op: the whole op on the chip route if the group's
 // blocks can hold the state, otherwise (a.staged) the staged route's clearing.
 // The later launches of an op that is over return at once.
-template <int KIND, bool C64>
+// STAGED: launches of the staged route follow.  OFF: the launch may be called off.
+template <int KIND, bool C64, bool STAGED, bool OFF>
 __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ OpSh sh;
   const int tid = threadIdx.x;
-  if (a.staged) {
+  if (STAGED && a.staged) {
     // too large for the chip route and accepted: as little code as can be (its
     // lines come from DRAM after an op on a large state)
     const long long n = a.in->nnz, nt = KIND == K_IDENT ? plain_tiles(n) : merge_tiles(n);
@@ -1808,28 +1809,28 @@ __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
     // descriptors, which block 0 rewrites at the end), the ones with a tile
     // at the others
     const int nact = n > 0 ? (int)((n + step - 1) / step) : 1;
-    Gate gate{word, nact, g.nblk, a.staged, 0u, false};
-    if (g.bid < nact) ok = op_chip<KIND, C64>(a, g, sh, X, gate, step, smem);
+    Gate gate{word, nact, g.nblk, 0u, false};
+    if (g.bid < nact) ok = op_chip<KIND, C64, OFF>(a, g, sh, X, gate, step, smem);
     else if (KIND != K_PERM) gate_arrive(gate);
     off = gate.off;
   } else {
     if (tid == 0) sh.R = OpResult{};
     if (g.bid == 0 && tid == 0) op_refuse(a, C64);
     // block 0 closes the op below: the others must have read its descriptors
-    Gate gate{word, 1, g.nblk, 0, 0u, false};
+    Gate gate{word, 1, g.nblk, 0u, false};
     gate_arrive(gate);
     if (g.bid == 0) ok = gate_wait(gate, a.ctrl);
   }
   pdl_trigger();
   if (g.bid == 0 && !off) {
-    if (a.staged && tid == 0) {  // for the launches that follow
+    if (STAGED && a.staged && tid == 0) {  // for the launches that follow
       stage_of(a)->state = ST_OVER;
       result_of(a)->failed = kOver;
     }
     // every block knows the result; the last one out only resets the barrier
     if (ok) op_close(a, KIND, P_GATHER, P_GATHER, sh.R, n);
   }
-  if (g.nblk > 1 && op_exit(a.ctrl, g.nblk, !ok && !off) == 3) {
+  if (g.nblk > 1 && op_exit(a.ctrl, g.nblk, !ok && !off) == 3 && OFF) {
     // called off: the staged launches do the op
     staged_zero(a, Grp{0, 1}, X.ntiles);
     if (tid == 0) stage_of(a)->state = ST_OK;
@@ -1908,7 +1909,7 @@ __device__ __forceinline__ void op_settle(const OpArgs& a, const Grp& g) {
   out_order_par(a.in, KIND, a.q, a.gb, sh.qat);
   __syncthreads();
   if (sh.St.state == ST_OVER) return;
-  Gate gate{reinterpret_cast<unsigned*>(&a.ctrl->sync_counter), g.nblk, g.nblk, 0, 0u, false};
+  Gate gate{reinterpret_cast<unsigned*>(&a.ctrl->sync_counter), g.nblk, g.nblk, 0u, false};
   unsigned phase = 0;
   const bool ok = sh.St.state != ST_GAVE_UP && staged_settle<KIND, C64>(a, g, sh, X, gate, &phase, smem);
   pdl_trigger();
@@ -1945,7 +1946,12 @@ __device__ __forceinline__ void op_write(const OpArgs& a, const Grp& g) {
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads, 4) k_op(const __grid_constant__ OpArgs a) {
   pdl_wait();
-  op_first<KIND, C64>(a, whole_grid());
+  op_first<KIND, C64, false, false>(a, whole_grid());
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op_try(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_first<KIND, C64, true, true>(a, whole_grid());
 }
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads) k_op_prep(const __grid_constant__ OpArgs a) {
@@ -1978,7 +1984,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const
   __shared__ OpArgs sa;
   pdl_wait();  // the plan is the kernel before's
   const Grp g = seg_enter(ops, plan, &sa, nullptr);
-  op_first<KIND, C64>(sa, g);
+  op_first<KIND, C64, true, false>(sa, g);
 }
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads) k_op_prep_seg(const OpArgs* ops, const SegPlan* plan) {
@@ -2019,11 +2025,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_write_seg(const OpArgs* ops,
 constexpr int kOpMaxBlocks = 1023;
 static_assert(kOpMaxBlocks <= (int)kExitMask && kOpMaxBlocks <= kMaxSets * 3 * 6, "block counts");
 
-// Resident grid of a kernel of kThreads threads (at most kOpMaxBlocks).
+// Resident grid of a kernel of kThreads threads (at most kOpMaxBlocks).  carveout:
+// the share of an SM's memory preferred as shared memory, in per cent.
 template <typename K>
-static cudaError_t op_grid(PerDevice& cache, K kern, size_t smem, int* grid) {
-  return per_device(cache, grid, [kern, smem](int* g) {
+static cudaError_t op_grid(PerDevice& cache, K kern, size_t smem, int* grid, int carveout = -1) {
+  return per_device(cache, grid, [kern, smem, carveout](int* g) {
     cudaError_t e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && carveout >= 0)
+      e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
     if (e != cudaSuccess) return e;
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem);
@@ -2039,15 +2048,22 @@ static cudaError_t op_grid(PerDevice& cache, K kern, size_t smem, int* grid) {
 struct OpGrids {
   int first, prep, eval, settle, write;
 };
+// (A staged op's first launch follows the write of the op before: the same split
+// of an SM's memory between L1 and shared memory spares it a change, 1 to 2 us
+// per op at 2^22 entries.)
+constexpr int kCarveout = 28;  // per cent: 64 KB
 template <int KIND, bool C64>
 static cudaError_t op_grids(OpGrids* g) {
-  static PerDevice cf, cp, ce, cs, cw;
+  static PerDevice cf, ct, cp, ce, cs, cw;
+  int unused = 0;
   cudaError_t e = op_grid(cf, k_op<KIND, C64>, kChipSmem, &g->first);
+  if constexpr (KIND != K_PERM)
+    if (e == cudaSuccess) e = op_grid(ct, k_op_try<KIND, C64>, kChipSmem, &unused, kCarveout);
   if (e == cudaSuccess) e = op_grid(cp, k_op_prep<KIND, C64>, 0, &g->prep);
   if (e == cudaSuccess) e = op_grid(ce, k_op_eval<KIND, C64>, kTileSmem, &g->eval);
   if constexpr (KIND != K_PERM) {
     if (e == cudaSuccess) e = op_grid(cs, k_op_settle<KIND, C64>, kTileSmem, &g->settle);
-    if (e == cudaSuccess) e = op_grid(cw, k_op_write<KIND, C64>, 0, &g->write);
+    if (e == cudaSuccess) e = op_grid(cw, k_op_write<KIND, C64>, 0, &g->write, kCarveout);
   }
   return e;
 }
@@ -2063,9 +2079,11 @@ static cudaError_t launch_op(OpArgs a, cudaStream_t s) {
   const long long want = bound <= kChipStep ? 1 : (bound + kChipMin - 1) / kChipMin;
   if (a.staged) g.first = KIND == K_IDENT ? device().sms : kFirstBlocks;
   else if (want < g.first) g.first = (int)want;
-  if (a.staged || g.first == 1) {  // no barrier, or one that may be called off
-    if (KIND != K_PERM || !a.staged)  // (a staged reorder has nothing to clear)
-      KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
+  if (a.staged) {
+    if constexpr (KIND != K_PERM)  // (a staged reorder has nothing to clear)
+      KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op_try<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
+  } else if (g.first == 1) {  // no barrier
+    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op<KIND, C64>, dim3(1), dim3(kThreads), kChipSmem, s, a));
   } else {
     KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
   }

@@ -362,7 +362,7 @@ __device__ __forceinline__ void tile_in_order(const TileSeg& T, const uint64_t* 
 template <int PT, int GB>
 __device__ __forceinline__ void tile_zorder(const TileSeg& T, const uint64_t* sK, uint16_t* sP, int* sWarp, int t) {
   const int E = (int)T.off[5];
-  if (t == GB) {
+  if (PT > 2 && t == GB) {  // (a chip tile's merge costs no more than the extra code)
     tile_in_order<PT, GB>(T, sK, sP);
     return;
   }
