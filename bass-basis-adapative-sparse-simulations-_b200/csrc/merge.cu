@@ -186,7 +186,7 @@ __device__ __forceinline__ void tile_body(const OpArgs& a, Grp g) {
     }
     __syncthreads();
     const int E = (int)T.off[5];
-    if (!tile_fetch<kPerThread, C64>(T, S, sZ, sA, &sBar, &phase, a.ctrl, kSpinLimit)) break;
+    if (!tile_fetch<kPerThread, C64>(T, S, sZ, sA, &sBar, &phase, a.ctrl, wait_limit(a.ctrl))) break;
     if (KIND != K_IDENT) tile_zorder<kPerThread, group_bit(KIND)>(T, sZ, sIdx, sWarp, t);
     const TileView V{sZ, sA, reinterpret_cast<const float2*>(sA), KIND == K_IDENT ? nullptr : sIdx, r0, r1, scaled, C64};
 
@@ -426,6 +426,7 @@ __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ Op
     const double2 v = C64 ? f2d(sAf[p]) : sA[p];
     return scaled ? amp_scale(v, C64 ? 1 : 0, r0, r1) : v;
   };
+  const long long lim = wait_limit(a.ctrl);
   __syncthreads();
   unsigned phase = 0;
   unsigned long long* item_ctr = &reinterpret_cast<unsigned long long*>(a.ws.counters)[a.counter];
@@ -450,12 +451,15 @@ __global__ void __launch_bounds__(kThreads) k_rdm_low(const __grid_constant__ Op
       if (tid == 0) copy_ragged(sK, keys, lo, hi, true);
       if (C64 && tid == 1) copy_ragged(sAf, ampf, lo, hi, true);
       bool done = false;
-      for (long long sp = 0; sp < kSpinLimit && !done; ++sp) done = mbar_try_wait(&sBar, phase);
-      phase ^= 1u;
+      for (long long sp = 0; sp < lim && !done; ++sp) done = mbar_try_wait(&sBar, phase);
       if (__syncthreads_or(!done)) {
         if (tid == 0) set_error(a.ctrl, BASS_ERR_WAIT);
+        // (the block must not end with its copies in flight)
+        for (long long sp = 0; sp < kSpinLimit && !done; ++sp) done = mbar_try_wait(&sBar, phase);
+        __syncthreads();
         break;
       }
+      phase ^= 1u;
     } else {
       for (int i = tid; i < E; i += kThreads) {
         sK[i] = keys[lo + i];
