@@ -45,11 +45,15 @@
 
 namespace bass {
 
-constexpr int kChipPT = 2;                       // entries per thread of a chip tile
-constexpr int kChipTile = kChipPT * kThreads;    // 512
-constexpr int kChipStep = kChipTile - 4;         // a boundary backs off by at most 4
+// Chip tiles of PT entries per thread: 2 (the smallest chains), or 4 for states
+// that only so fit the chip.
+template <int PT>
+constexpr int kChipTile = PT * kThreads;         // 512, 1024
+template <int PT>
+constexpr int kChipStep = kChipTile<PT> - 4;     // a boundary backs off by at most 4
 constexpr int kChipMin = 252;                    // smallest tile step when the grid would allow less
-constexpr int kChipPad = kChipTile + 8;
+template <int PT>
+constexpr int kChipPad = kChipTile<PT> + 8;
 constexpr int kChipBins = 2048;                  // digits of the chip search: 11 bits (the first: the exponent)
 constexpr int kChipLate = 32;                    // undecided children it stops at (one per lane of a warp)
 constexpr int kSelMax = 256;                     // boundary children settled by ranking (one per thread)
@@ -78,8 +82,10 @@ static_assert(kListAt + 3 * kSelMax <= 2 * 1024, "the list fits ws.red");
 // dynamic shared memory: a staged tile; a chip tile plus the histogram (which
 // the settled children share)
 constexpr size_t kTileSmem = (size_t)kTilePad * (16 + 8 + 2);
-constexpr size_t kChipHistAt = ((size_t)kChipPad * (16 + 8 + 2) + 127) & ~(size_t)127;
-constexpr size_t kChipSmem = kChipHistAt + (size_t)kChipBins * 4;
+template <int PT>
+constexpr size_t kChipHistAt = ((size_t)kChipPad<PT> * (16 + 8 + 2) + 127) & ~(size_t)127;
+template <int PT>
+constexpr size_t kChipSmem = kChipHistAt<PT> + (size_t)kChipBins * 4;
 
 // ---------------------------------------------------------------------------
 // grid barriers
@@ -568,7 +574,7 @@ struct OpSh {
   unsigned long long limb[8];
   i128 red[2 * kRegions];
   long long sum[5 * kRegions];  // block_sum's
-  int warp[2 * kRegions];
+  int warp[4 * kRegions];
   uint64_t bar;
   long long item;
   int8_t qat[64];  // output qubit order
@@ -679,20 +685,19 @@ __device__ __forceinline__ void flush_sums(OpSh& sh, unsigned long long* cn, i12
 // ---- chip route -------------------------------------------------------------
 // Block b of nact holds tile b (step Z positions).  Returns false if a wait
 // gave up; otherwise sh.R is the op's result.
-template <int KIND, bool C64, bool OFF>
+template <int KIND, bool C64, bool OFF, int PT>
 __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh, const OpCtx& X, Gate& gate, int step,
                                         unsigned char* smem) {
   constexpr int NS = slots_per_entry(KIND);
-  constexpr int PT = kChipPT;
   constexpr bool P2 = KIND == K_ROT1;  // rotation steps: sums of |a|^2 and |a|^4; others: kept and total |a|^2
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   double2* sA = reinterpret_cast<double2*>(smem);
-  uint64_t* sZ = reinterpret_cast<uint64_t*>(sA + kChipPad);
-  uint16_t* sIdx = reinterpret_cast<uint16_t*>(sZ + kChipPad);
-  unsigned* sHist = reinterpret_cast<unsigned*>(smem + kChipHistAt);
+  uint64_t* sZ = reinterpret_cast<uint64_t*>(sA + kChipPad<PT>);
+  uint16_t* sIdx = reinterpret_cast<uint16_t*>(sZ + kChipPad<PT>);
+  unsigned* sHist = reinterpret_cast<unsigned*>(smem + kChipHistAt<PT>);
   CandSh& sCand = *reinterpret_cast<CandSh*>(sHist);                              // after the search
   uint8_t* sKeep = reinterpret_cast<uint8_t*>(sHist) + ((sizeof(CandSh) + 15) & ~15);  // per position, settled children
-  static_assert(((sizeof(CandSh) + 15) & ~15) + kChipTile <= 4 * kChipBins, "the settled children fit the histogram");
+  static_assert(((sizeof(CandSh) + 15) & ~15) + kChipTile<PT> <= 4 * kChipBins, "the settled children fit the histogram");
   const bool multi = gate.nact > 1;
   const int nact = gate.nact;
   const long long n = X.S.n;
@@ -730,7 +735,7 @@ __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh,
   }
   __syncthreads();
   if (tid == 0)
-    tile_segments<C64>(sh.T, sh.rec[0], sh.rec[1], X.S, kChipTile, sZ, sA, &sh.bar, a.ctrl);
+    tile_segments<C64>(sh.T, sh.rec[0], sh.rec[1], X.S, kChipTile<PT>, sZ, sA, &sh.bar, a.ctrl);
   if (KIND != K_PERM && X.may_trunc)
     for (int i = tid; i < kChipBins; i += kThreads) sHist[i] = 0u;
   __syncthreads();
@@ -866,7 +871,7 @@ __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh,
   }
   s0.fold();
   s1.fold();
-  // at most 8 terms below 1 per thread: the block's integers fit 64 bits
+  // at most 16 terms below 1 per thread: the block's integers fit 64 bits
   long long bs[5] = {nkeep, s0.ih, s0.il, s1.ih, s1.il};
   if (sums) {
     block_sum<5>(bs, sh.sum);
@@ -903,7 +908,7 @@ __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh,
   }
   if (cut.late) {
     const int m = load_cands(list, cn, sCand);
-    for (int i = tid; i < kChipTile / 4; i += kThreads) reinterpret_cast<unsigned*>(sKeep)[i] = 0u;
+    for (int i = tid; i < kChipTile<PT> / 4; i += kThreads) reinterpret_cast<unsigned*>(sKeep)[i] = 0u;
     __syncthreads();
     if (rank_cand(sCand, m, cut.need)) {
       const unsigned long long b = sCand.bits[tid];
@@ -987,10 +992,11 @@ __device__ __forceinline__ bool op_chip(const OpArgs& a, const Grp& g, OpSh& sh,
 }
 
 // The tile step of a chip op on nblk blocks, or 0 if they cannot hold it.
+template <int PT>
 __device__ __forceinline__ int chip_step(long long n, int nblk) {
-  if (n <= kChipStep) return kChipStep;
+  if (n <= kChipStep<PT>) return kChipStep<PT>;
   const long long step = ((n + nblk - 1) / nblk + 3) & ~3LL;
-  return step > kChipStep ? 0 : step < kChipMin ? kChipMin : (int)step;
+  return step > kChipStep<PT> ? 0 : step < kChipMin ? kChipMin : (int)step;
 }
 
 // ---- staged route -------------------------------------------------------------
@@ -1127,7 +1133,8 @@ __device__ __forceinline__ void staged_prep(const OpArgs& a, const Grp& g, const
   if (KIND != K_IDENT) {
     for (long long b = gtid >> 5; b <= X.ntiles; b += gthreads >> 5) {
       long long r[6];
-      tile_boundary<group_bit(KIND)>(X.S.keys, n, b * kStep, X.t, KIND != K_PERM, r);
+      if (X.t == group_bit(KIND)) low_boundary<group_bit(KIND)>(X.S.keys, n, b * kStep, KIND != K_PERM, r);
+      else tile_boundary<group_bit(KIND)>(X.S.keys, n, b * kStep, X.t, KIND != K_PERM, r);
       if ((threadIdx.x & 31) == 0)
         for (int q = 0; q < 6; ++q) a.ws.part[b * 6 + q] = r[q];
     }
@@ -1777,7 +1784,7 @@ __device__ __forceinline__ void op_close(const OpArgs& a, int kind, int pass_in,
 // blocks can hold the state, otherwise (a.staged) the staged route's clearing.
 // The later launches of an op that is over return at once.
 // STAGED: launches of the staged route follow.  OFF: the launch may be called off.
-template <int KIND, bool C64, bool STAGED, bool OFF>
+template <int KIND, bool C64, bool STAGED, bool OFF, int PT>
 __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ OpSh sh;
@@ -1786,7 +1793,7 @@ __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
     // too large for the chip route and accepted: as little code as can be (its
     // lines come from DRAM after an op on a large state)
     const long long n = a.in->nnz, nt = KIND == K_IDENT ? plain_tiles(n) : merge_tiles(n);
-    if (n > (long long)g.nblk * kChipStep && n * slots_per_entry(KIND) <= a.ws.max_n && nt <= a.ws.max_tiles &&
+    if (n > (long long)g.nblk * kChipStep<PT> && n * slots_per_entry(KIND) <= a.ws.max_n && nt <= a.ws.max_tiles &&
         n < kMaxEntries && (a.in->amp_type == BASS_AMP_C64) == C64) {
       pdl_trigger();
       staged_zero(a, g, nt);
@@ -1796,7 +1803,7 @@ __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
   }
   const OpCtx X = op_ctx<KIND, C64>(a);
   const long long n = X.S.n;
-  const int step = X.bad ? 0 : chip_step(n, g.nblk);
+  const int step = X.bad ? 0 : chip_step<PT>(n, g.nblk);
   if (tid == 0) mbar_init(&sh.bar, 1);
   out_order_par(a.in, KIND, a.q, a.gb, sh.qat);
   __syncthreads();
@@ -1810,7 +1817,7 @@ __device__ __forceinline__ void op_first(const OpArgs& a, const Grp& g) {
     // at the others
     const int nact = n > 0 ? (int)((n + step - 1) / step) : 1;
     Gate gate{word, nact, g.nblk, 0u, false};
-    if (g.bid < nact) ok = op_chip<KIND, C64, OFF>(a, g, sh, X, gate, step, smem);
+    if (g.bid < nact) ok = op_chip<KIND, C64, OFF, PT>(a, g, sh, X, gate, step, smem);
     else if (KIND != K_PERM) gate_arrive(gate);
     off = gate.off;
   } else {
@@ -1946,12 +1953,17 @@ __device__ __forceinline__ void op_write(const OpArgs& a, const Grp& g) {
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads, 4) k_op(const __grid_constant__ OpArgs a) {
   pdl_wait();
-  op_first<KIND, C64, false, false>(a, whole_grid());
+  op_first<KIND, C64, false, false, 2>(a, whole_grid());
+}
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op4(const __grid_constant__ OpArgs a) {
+  pdl_wait();
+  op_first<KIND, C64, false, false, 4>(a, whole_grid());
 }
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads, 4) k_op_try(const __grid_constant__ OpArgs a) {
   pdl_wait();
-  op_first<KIND, C64, true, true>(a, whole_grid());
+  op_first<KIND, C64, true, true, 2>(a, whole_grid());
 }
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads) k_op_prep(const __grid_constant__ OpArgs a) {
@@ -1984,7 +1996,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_op_seg(const OpArgs* ops, const
   __shared__ OpArgs sa;
   pdl_wait();  // the plan is the kernel before's
   const Grp g = seg_enter(ops, plan, &sa, nullptr);
-  op_first<KIND, C64, true, false>(sa, g);
+  op_first<KIND, C64, false, false, 2>(sa, g);
+}
+// (states that need larger tiles, or the launches after this one)
+template <int KIND, bool C64>
+__global__ void __launch_bounds__(kThreads, 4) k_op4_seg(const OpArgs* ops, const SegPlan* plan) {
+  __shared__ OpArgs sa;
+  pdl_wait();
+  const Grp g = seg_enter(ops, plan, &sa, nullptr);
+  op_first<KIND, C64, true, false, 4>(sa, g);
 }
 template <int KIND, bool C64>
 __global__ void __launch_bounds__(kThreads) k_op_prep_seg(const OpArgs* ops, const SegPlan* plan) {
@@ -2044,9 +2064,17 @@ static cudaError_t op_grid(PerDevice& cache, K kern, size_t smem, int* grid, int
   });
 }
 
+// The kinds that take states of up to 592 x 1020 entries on chip, in larger tiles
+// (us per op of 400,000 entries, staged and on chip: 1-qubit gate 73 and 56,
+// 2-qubit gate 119 and 107, truncation 52 and 39; of 600,000: 81 and 60, 130 and
+// 124, 58 and 52).  A rotation step that is rejected writes nothing, and the
+// larger tiles' chain costs more than the staging: 67 and 71, 74 and 79.
+template <int KIND>
+constexpr bool kChip4 = KIND != K_PERM && KIND != K_ROT1;
+
 // The grids of a kind's launches.
 struct OpGrids {
-  int first, prep, eval, settle, write;
+  int first, first4, prep, eval, settle, write;
 };
 // (A staged op's first launch follows the write of the op before: the same split
 // of an SM's memory between L1 and shared memory spares it a change, 1 to 2 us
@@ -2054,11 +2082,14 @@ struct OpGrids {
 constexpr int kCarveout = 28;  // per cent: 64 KB
 template <int KIND, bool C64>
 static cudaError_t op_grids(OpGrids* g) {
-  static PerDevice cf, ct, cp, ce, cs, cw;
+  static PerDevice cf, c4, ct, cp, ce, cs, cw;
   int unused = 0;
-  cudaError_t e = op_grid(cf, k_op<KIND, C64>, kChipSmem, &g->first);
-  if constexpr (KIND != K_PERM)
-    if (e == cudaSuccess) e = op_grid(ct, k_op_try<KIND, C64>, kChipSmem, &unused, kCarveout);
+  cudaError_t e = op_grid(cf, k_op<KIND, C64>, kChipSmem<2>, &g->first);
+  if constexpr (kChip4<KIND>)
+    if (e == cudaSuccess) e = op_grid(c4, k_op4<KIND, C64>, kChipSmem<4>, &g->first4);
+  if constexpr (KIND != K_PERM) {
+    if (e == cudaSuccess) e = op_grid(ct, k_op_try<KIND, C64>, kChipSmem<2>, &unused, kCarveout);
+  }
   if (e == cudaSuccess) e = op_grid(cp, k_op_prep<KIND, C64>, 0, &g->prep);
   if (e == cudaSuccess) e = op_grid(ce, k_op_eval<KIND, C64>, kTileSmem, &g->eval);
   if constexpr (KIND != K_PERM) {
@@ -2075,17 +2106,23 @@ static cudaError_t launch_op(OpArgs a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   // the workspace bounds the entries (the kernels refuse more)
   const long long bound = a.ws.max_n / slots_per_entry(KIND);
-  a.staged = bound > (long long)g.first * kChipStep;
-  const long long want = bound <= kChipStep ? 1 : (bound + kChipMin - 1) / kChipMin;
+  const bool larger = bound > (long long)g.first * kChipStep<2>;
+  a.staged = larger && (!kChip4<KIND> || bound > (long long)g.first4 * kChipStep<4>);
+  const long long want = bound <= kChipStep<2> ? 1 : (bound + kChipMin - 1) / kChipMin;
   if (a.staged) g.first = KIND == K_IDENT ? device().sms : kFirstBlocks;
   else if (want < g.first) g.first = (int)want;
   if (a.staged) {
     if constexpr (KIND != K_PERM)  // (a staged reorder has nothing to clear)
-      KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op_try<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
+      KLAUNCH(KIND * 5 + P_GATHER, s,
+              e = launch_pdl(k_op_try<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem<2>, s, a));
+  } else if (larger) {
+    if constexpr (kChip4<KIND>)
+      KLAUNCH(KIND * 5 + P_GATHER, s,
+              e = launch_coop(k_op4<KIND, C64>, dim3(g.first4), dim3(kThreads), kChipSmem<4>, s, a));
   } else if (g.first == 1) {  // no barrier
-    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op<KIND, C64>, dim3(1), dim3(kThreads), kChipSmem, s, a));
+    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_pdl(k_op<KIND, C64>, dim3(1), dim3(kThreads), kChipSmem<2>, s, a));
   } else {
-    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, a));
+    KLAUNCH(KIND * 5 + P_GATHER, s, e = launch_coop(k_op<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem<2>, s, a));
   }
   if (e != cudaSuccess || !a.staged) return e;
   KLAUNCH(S_PARTITION, s, e = launch_pdl(k_op_prep<KIND, C64>, dim3(g.prep), dim3(kThreads), 0, s, a));
@@ -2111,14 +2148,15 @@ cudaError_t merge_op(const OpArgs& a, cudaStream_t s) {
 template <int KIND, bool C64>
 static cudaError_t seg_op_grid(int* grid) {
   static PerDevice cache;
-  return op_grid(cache, k_op_seg<KIND, C64>, kChipSmem, grid);
+  return op_grid(cache, k_op_seg<KIND, C64>, kChipSmem<2>, grid);
 }
 
 // Do the staged launches have to follow the first one?  Not if every state fits
 // its blocks however many entries it holds: with work weights n + kSegPad a
 // state gets more than (grid - nseg) (n + kSegPad) / W blocks, so W <= (grid -
-// nseg) kChipStep, which the workspaces' bounds show, is enough.  slots: children
-// per entry that the workspaces are sized for.
+// nseg) kChipStep, which the workspaces' bounds show, is enough: 0 for the small
+// tiles, 1 for the larger ones; 2 otherwise.  slots: children per entry that the
+// workspaces are sized for.
 template <int KIND>
 cudaError_t seg_stages_t(OpArgs* ops, int nseg, int slots, int* staged) {
   int grid = 0;
@@ -2126,17 +2164,19 @@ cudaError_t seg_stages_t(OpArgs* ops, int nseg, int slots, int* staged) {
   if (e != cudaSuccess) return e;
   long long w = 0;
   for (int i = 0; i < nseg; ++i) w += ops[i].ws.max_n / slots + kSegPad;
-  *staged = w > (long long)(grid - nseg) * kChipStep;
-  for (int i = 0; i < nseg; ++i) ops[i].staged = *staged, ops[i].seg = 1;
+  const long long fit = w / (grid - nseg > 0 ? grid - nseg : 1);
+  *staged = fit < kChipStep<2> ? 0 : fit < kChipStep<4> ? 1 : 2;
+  for (int i = 0; i < nseg; ++i) ops[i].staged = *staged == 2, ops[i].seg = 1;
   return cudaSuccess;
 }
 
 // The first launch is cooperative, since states that stay on chip share it.
 template <int KIND, bool C64>
 static cudaError_t merge_op_seg(const OpArgs* ops, int nseg, int staged, SegPlan* plan, cudaStream_t s) {
-  static PerDevice cp, ce, cs, cw;
+  static PerDevice c4, cp, ce, cs, cw;
   OpGrids g{};
   cudaError_t e = seg_op_grid<KIND, C64>(&g.first);
+  if (e == cudaSuccess) e = op_grid(c4, k_op4_seg<KIND, C64>, kChipSmem<4>, &g.first4);
   if (e == cudaSuccess) e = op_grid(cp, k_op_prep_seg<KIND, C64>, 0, &g.prep);
   if (e == cudaSuccess) e = op_grid(ce, k_op_eval_seg<KIND, C64>, kTileSmem, &g.eval);
   if constexpr (KIND != K_PERM) {
@@ -2149,9 +2189,13 @@ static cudaError_t merge_op_seg(const OpArgs* ops, int nseg, int staged, SegPlan
   if (nseg > most) return cudaErrorInvalidValue;
   if ((e = run_seg_plan(ops, nseg, KIND, plan, s)) != cudaSuccess) return e;
   const SegPlan* p = plan;
-  KLAUNCH(KIND * 5 + P_GATHER, s,
-          e = launch_coop(k_op_seg<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem, s, ops, p));
-  if (e != cudaSuccess || !staged) return e;
+  if (staged == 0)
+    KLAUNCH(KIND * 5 + P_GATHER, s,
+            e = launch_coop(k_op_seg<KIND, C64>, dim3(g.first), dim3(kThreads), kChipSmem<2>, s, ops, p));
+  else
+    KLAUNCH(KIND * 5 + P_GATHER, s,
+            e = launch_coop(k_op4_seg<KIND, C64>, dim3(g.first4), dim3(kThreads), kChipSmem<4>, s, ops, p));
+  if (e != cudaSuccess || staged < 2) return e;
   KLAUNCH(S_PARTITION, s, e = launch_pdl(k_op_prep_seg<KIND, C64>, dim3(g.prep), dim3(kThreads), 0, s, ops, p));
   if (e != cudaSuccess) return e;
   KLAUNCH(KIND * 5 + P_HIST, s,

@@ -101,6 +101,33 @@ __device__ __forceinline__ void tile_boundary(const uint64_t* keys, long long n,
   r[0] = s + i + j; r[1] = s; r[2] = mid; r[3] = e; r[4] = i; r[5] = j;
 }
 
+// tile_boundary when the target bit is already in its place (t == GB): a block is
+// a group, at most 2 << GB entries around P, so one load replaces the searches.
+template <int GB>
+__device__ __forceinline__ void low_boundary(const uint64_t* keys, long long n, long long P, bool back,
+                                             long long (&r)[6]) {
+  if (P >= n) {
+    r[0] = n; r[1] = n; r[2] = n; r[3] = n; r[4] = 0; r[5] = 0;
+    return;
+  }
+  constexpr int kReach = (2 << GB) - 1;
+  const int lane = threadIdx.x & 31;
+  const uint64_t y = keys[P];
+  const long long p = P - kReach + lane;
+  const bool in = lane <= 2 * kReach && p >= 0 && p < n;
+  const uint64_t k = in ? keys[p] : 0ULL;
+  const bool mine = in && (k >> (GB + 1)) == (y >> (GB + 1));
+  const unsigned m = __ballot_sync(0xffffffffu, mine), m1 = __ballot_sync(0xffffffffu, mine && ((k >> GB) & 1ULL));
+  const long long s = P - kReach + (__ffs(m) - 1), e = s + __popc(m), mid = e - __popc(m1);
+  long long i = 0, j = 0;
+  if (!back) {
+    const long long d = P - s, len0 = mid - s;
+    i = d < len0 ? d : len0;
+    j = d - i;
+  }
+  r[0] = s + i + j; r[1] = s; r[2] = mid; r[3] = e; r[4] = i; r[5] = j;
+}
+
 // ---------------------------------------------------------------------------
 // a tile's input
 // ---------------------------------------------------------------------------
@@ -327,11 +354,13 @@ __device__ __forceinline__ void tile_merge(const TileSeg& T, const uint64_t* sK,
   }
   if (LISTS) __syncthreads();  // the lists are read before they are overwritten
   // consecutive positions in one store (what lies past E is never read)
-  static_assert(PT == 8 || PT == 2, "write-back of eight or two positions");
+  static_assert(PT == 8 || PT == 4 || PT == 2, "write-back of eight, four or two positions");
   if (tid * PT < E) {
     if (PT == 8)
       *reinterpret_cast<uint4*>(sP + d) = make_uint4(rp[0] | (rp[1] << 16), rp[2 % PT] | (rp[3 % PT] << 16),
                                                      rp[4 % PT] | (rp[5 % PT] << 16), rp[6 % PT] | (rp[7 % PT] << 16));
+    else if (PT == 4)
+      *reinterpret_cast<uint2*>(sP + d) = make_uint2(rp[0] | (rp[1] << 16), rp[2 % PT] | (rp[3 % PT] << 16));
     else
       *reinterpret_cast<unsigned*>(sP + d) = rp[0] | (rp[1] << 16);
   }

@@ -24,7 +24,7 @@ def _state(n, dtype, seed):
     return st, x, a
 
 
-@pytest.mark.parametrize("n", [3, 507, 5001, 330001])
+@pytest.mark.parametrize("n", [3, 507, 5001, 330001, 620001])
 def test_lowest_bits_match_oracle(pkg, orc, n):
     from bass_b200 import _native as nat
     from bass_b200.gates import haar_random_unitary
@@ -49,7 +49,7 @@ def test_lowest_bits_match_oracle(pkg, orc, n):
         assert abs(np.trace(rho) - np.sum(np.abs(a) ** 2)) < 1e-9
 
 
-@pytest.mark.parametrize("n", [507, 5001, 330001])
+@pytest.mark.parametrize("n", [507, 5001, 330001, 620001])
 def test_lowest_bits_complex64(pkg, n):
     """complex64: the same gate on a qubit that is merged and on the same
     entries with that qubit renamed to the lowest bit."""

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 EVAL, CHIP, WRITE = 0, 2, 3   # passes of an op kind's slots
 
 
-@pytest.mark.parametrize("n,read,wrote", [(400, CHIP, CHIP), (5000, CHIP, CHIP), (400000, EVAL, WRITE)])
+@pytest.mark.parametrize("n,read,wrote", [(400, CHIP, CHIP), (5000, CHIP, CHIP), (400000, CHIP, CHIP), (620000, EVAL, WRITE)])
 @pytest.mark.parametrize("op,kind", [("gate1", 0), ("gate2", 2), ("topk", 4)])
 def test_entries_are_counted_where_they_move(pkg, n, read, wrote, op, kind):
     from bass_b200 import _native as nat

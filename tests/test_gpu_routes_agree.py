@@ -58,7 +58,7 @@ def _run(x, a, op, k, bound, offset):
     from bass_b200.gates import haar_random_unitary
     from bass_b200.state import SparseState
     G1, G2 = haar_random_unitary(2, seed=2), haar_random_unitary(4, seed=3)
-    st = SparseState(N, 1 << 17, dtype=a.dtype, _capacity=1 << 19)
+    st = SparseState(N, 1 << 17, dtype=a.dtype, _capacity=1 << 20)
     st.load(x, a)
     eng, cur = st._eng, st._cur
     keep = None

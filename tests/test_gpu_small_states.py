@@ -22,7 +22,7 @@ def _state(n, seed, dtype=np.complex128):
     x = np.sort(rng.permutation(x)[:n])
     a = rng.standard_normal(n) + 1j * rng.standard_normal(n)
     a = (a / np.linalg.norm(a)).astype(dtype)
-    st = SparseState(N, 1 << 19, dtype=dtype, _capacity=1 << 19)
+    st = SparseState(N, 1 << 20, dtype=dtype, _capacity=1 << 20)
     st.load(x, a)
     st._cur.nmax = st._cur.cap       # as after gates that were not truncated
     return st, x, a

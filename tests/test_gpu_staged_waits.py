@@ -13,7 +13,7 @@ def test_staged_op_gives_up_and_recovers(pkg, orc, op):
     from bass_b200 import _native as nat
     from bass_b200.gates import haar_random_unitary
     from bass_b200.state import SparseState
-    N, n, k = 32, 400000, 250000
+    N, n, k = 32, 620000, 400000
     rng = np.random.default_rng(5)
     x = np.unique(rng.integers(0, 2 ** N, size=n + 200, dtype=np.uint64))[:n]
     a = rng.standard_normal(n) + 1j * rng.standard_normal(n)
