@@ -52,12 +52,12 @@ PROF_SLOTS = 48
 KINDS = ["gate1", "rot1", "gate2", "perm", "plain", "rdm"]
 PASSES = ["hist", "hist2", "gather", "write", "rdm"]
 SLOT_NAMES = [f"k_tile<{k},{p}>" for k in KINDS for p in PASSES] + [
-    "k_partition", "k_op_zero", "unused32", "unused33", "unused34", "reductions", "k_fingerprint",
+    "k_partition", "unused31", "unused32", "unused33", "unused34", "reductions", "k_fingerprint",
     "k_phase2q", "k_phase1q", "k_rdm_final", "radix_sort", "merge_runs", "bookkeeping", "unused43",
     "unused44", "unused45", "unused46", "unused47"]
 # gates, rotation steps, truncations and reorders: the staged route's passes
-# (its tile boundaries and sample are in the partition's slot), and the chip
-# route's one launch
+# (its tile boundaries and sample are in the partition's slot), and the first
+# launch, a chip op's only one
 for _k, _name in enumerate(KINDS[:5]):
     SLOT_NAMES[5 * _k] = f"k_op_eval<{_name}>"
     SLOT_NAMES[5 * _k + 1] = f"k_op_settle<{_name}>"

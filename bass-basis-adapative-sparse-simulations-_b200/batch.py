@@ -87,8 +87,8 @@ class StatePool:
         # every slot's control block and RDM moments are contiguous: one read covers them all
         self.ctrl_all = torch.zeros((S, cb), dtype=torch.uint8, device=self.device)
         self.rho_all = torch.zeros((S, 4 * 64), dtype=torch.float64, device=self.device)
-        # a segmented selection keeps one block group per state resident: a
-        # launch takes at most this many states (one selection block per SM)
+        # an op's grid barriers keep every block group resident: a launch takes
+        # at most this many states (one per SM)
         self.seg_chunk = max(1, min(MAX_SEG, int(self.L.bass_batch_max_segments())))
         self.bws_bytes = int(self.L.bass_batch_ws_bytes(self.seg_chunk))
         self.bws = torch.empty(self.bws_bytes, dtype=torch.uint8, device=self.device)

@@ -66,8 +66,6 @@ const Device& device() {
     if (dev < kMaxDevices) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     x.sms = sms > 0 ? sms : 1;
     x.grid_small = x.sms * 8;
-    x.grid_tile = x.sms * 2;
-    x.grid_tile_h = x.sms;
     d[dev] = x;
   });
   return d[dev];

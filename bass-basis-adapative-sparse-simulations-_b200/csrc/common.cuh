@@ -88,10 +88,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
-// A hint: bring [src, src + bytes) into L2 (no completion to wait for).
-__device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 
 // ---------------------------------------------------------------------------
 // exact accumulation
@@ -426,12 +422,6 @@ __device__ __forceinline__ void warp_lower_bound3(const uint64_t* keys, long lon
 // this block's part of the grid no longer needs its SM to itself, so the next
 // kernel may be scheduled.  Both are no-ops for a kernel launched normally.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Nanosecond wall clock of the GPU (profiling of phases inside one launch).
-__device__ __forceinline__ unsigned long long gtimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // One galloping round before warp_lower_bound3, for three searches whose
@@ -587,8 +577,6 @@ __host__ __device__ __forceinline__ long long plain_tiles(long long n) { return 
 
 struct Partial {
   i128 s[4];
-  long long c[2];
-  long long pad[2];
 };
 
 // What later launches read of an op.
@@ -601,7 +589,6 @@ struct SelState {
   long long n_written;
   double kept;           // exact sum of |a|^2 over the kept children
   int accept;            // rotation step: the candidate lowers PR
-  int unused;
   double pr_new;         // rotation step: PR of the candidate
 };
 
@@ -620,7 +607,7 @@ struct WsView {
   double2* tmp_amps;             // staged amplitudes; max_n: second amplitude buffer
   uint64_t* stage_keys;          // staged keys
   uint8_t* kmask;                // kept bits of the staged children, NS 8 words per region
-  unsigned int* sort_hist;       // radix-sort tile histograms (256 x max_tiles)
+  unsigned int* sort_hist;       // the sort's look-back words (256 of 8 bytes per tile of 4096)
   i128* red;                     // 1024 per-CTA reduction partials
   unsigned long long* fp;        // 8 fingerprint accumulators
   long long max_n;

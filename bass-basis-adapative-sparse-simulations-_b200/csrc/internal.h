@@ -13,7 +13,7 @@ namespace bass {
 
 enum Kind { K_GATE1 = 0, K_ROT1 = 1, K_GATE2 = 2, K_PERM = 3, K_IDENT = 4, K_RDM = 5 };
 // Profile slots of a kind (kind * 5 + pass): P_HIST the staged evaluation,
-// P_HIST2 its settling, P_GATHER the chip route's one launch, P_WRITE the write
+// P_HIST2 its settling, P_GATHER the first launch (a chip op's only one), P_WRITE the write
 // (and the compaction after a diagonal 1-qubit gate), P_RDM moments.
 enum Pass { P_HIST = 0, P_HIST2 = 1, P_GATHER = 2, P_WRITE = 3, P_RDM = 4 };
 
@@ -58,7 +58,7 @@ struct SegPlan {
 constexpr int kSegPad = 252;
 
 enum Slot {
-  S_PARTITION = 30, S_ZERO = 31, S_REDUCE = 35,
+  S_PARTITION = 30, S_REDUCE = 35,
   S_FINGERPRINT = 36, S_PHASE2Q = 37, S_PHASE1Q = 38, S_RDM_FINAL = 39, S_SORT = 40, S_MERGE_RUNS = 41,
   S_SMALL = 42
 };
@@ -102,8 +102,6 @@ inline cudaError_t launch_pdl(void (*kern)(K...), dim3 grid, dim3 block, size_t 
 
 struct Device {
   int sms;
-  int grid_tile;    // persistent grid of the tile kernels
-  int grid_tile_h;  // ... of the histogram passes (more shared memory)
   int grid_small;
 };
 // The current device's properties (looked up once per device).
@@ -157,8 +155,8 @@ cudaError_t run_ident_write(OpArgs a, cudaStream_t s);
 cudaError_t run_commit(bass_state* cur, bass_state* tmp, bass_ctrl* ctrl, const WsView& ws, int j, int trace,
                        cudaStream_t s);
 
-// merge.cu, segmented: ops_dev holds nseg OpArgs (all of one amplitude type),
-// plan_dev is scratch for the block groups
+// op.cu and merge.cu, segmented: ops_dev holds nseg OpArgs (all of one amplitude
+// type), plan_dev is scratch for the block groups
 cudaError_t run_merge_op_seg(int kind, const OpArgs* ops_dev, int nseg, int c64, int staged, SegPlan* plan_dev,
                              cudaStream_t s);
 // sets the ops' launches (OpArgs::staged) before they are copied to the device

@@ -15,8 +15,8 @@ namespace bass {
 // ---------------------------------------------------------------------------
 // partition
 // ---------------------------------------------------------------------------
-// The op's small workspace region (tile counters, histograms, selection
-// state, look-back status words: what zero_small clears), zeroed by a group.
+// The small workspace region (tile counters, histograms, SelState, look-back
+// status words: what zero_small clears), zeroed by a group.
 __device__ __forceinline__ void zero_op_region(const OpArgs& a, Grp g) {
   unsigned long long* zp = reinterpret_cast<unsigned long long*>(a.ws.counters);
   const long long nw =

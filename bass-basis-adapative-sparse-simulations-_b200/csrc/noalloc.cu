@@ -14,7 +14,7 @@
 //     a state that does not fit the scratch although max_entries said it
 //     would is refused by the kernels themselves (BASS_ERR_WORKSPACE in ctrl,
 //     NaN in rho);
-//   * the array (about 4.8 MB) is part of the library image: every GPU that
+//   * the array (about 3.7 MB) is part of the library image: every GPU that
 //     loads the library holds it until the process exits;
 //   * all calls share the one array: calls that may overlap on the GPU (other
 //     streams, other host threads) race and must be serialised by the caller;
@@ -76,7 +76,7 @@ extern "C" int bass_rdm_1q_noalloc(const bass_state* st, int64_t max_entries, in
   NoAllocScratch* sc = nullptr;
   if (noalloc_scratch(&sc) != cudaSuccess) return BASS_ERR_CUDA;
   cudaStream_t s = (cudaStream_t)stream;
-  // the tile counters and the selection state must start at zero
+  // the tile counters and the SelState must start at zero
   cudaError_t e = cudaMemsetAsync(sc, 0, offsetof(NoAllocScratch, part), s);
   if (e != cudaSuccess) return BASS_ERR_CUDA;
   WsView v{};

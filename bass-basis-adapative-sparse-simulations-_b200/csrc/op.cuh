@@ -2,17 +2,16 @@
 //
 // An op reads a sorted state in Z order (tile.cuh), evaluates the children of
 // every group, keeps the k of largest |a|^2 (ties: smaller true key) and writes
-// them, sorted again, with the bookkeeping of the truncation.  Two routes; the
-// host takes the first whenever the workspace bounds the state's entries by
-// what it can hold (launch_op):
+// them, sorted again, with the bookkeeping of the truncation.  Two routes:
 //
 //   chip    one cooperative launch.  Every block holds its tile in shared
 //           memory from the load to the write, so nothing is staged, and the
 //           threshold search works on |a|^2 held in registers, with a grid
 //           barrier per step.  What bounds it is latency, so tiles are small
-//           (252 to 508 entries), the grid is no larger than the bound asks,
-//           and only blocks that have a tile take part in the barriers: a state
-//           of up to 508 entries is one block's, without any.
+//           (252 to 508 entries; up to 1020 for gates and truncations of states
+//           that only so fit), the grid is no larger than the bound asks, and
+//           only blocks that have a tile take part in the barriers: a state of
+//           up to 508 entries is one block's, without any.
 //   staged  larger states: a sample of the children brackets the threshold
 //           first; the evaluation then stages only the children at or above the
 //           bracket (the ones certainly kept, and the few per cent inside it),
@@ -21,22 +20,29 @@
 //           What bounds it is instruction issue in the evaluation and memory
 //           traffic in the copy; the passes are launches of their own so that
 //           each has the registers it needs (as one kernel of barriers the
-//           evaluation spilled: 142 us instead of 93 at 2^22 entries).  A bracket that
-//           missed the threshold (seen from exact counts) is replaced by the
+//           evaluation spilled: 142 us instead of 93 at 2^22 entries).  A bracket
+//           that missed the threshold (seen from exact counts) is replaced by the
 //           exact one and the evaluation repeated: the result never depends on
 //           the sample.
+//
+// The host takes the chip route when the workspace bounds the state's entries by
+// what it holds (launch_op); under a larger bound the staged route's first launch
+// does the whole op if the state turns out small, and the others return at once.
 //
 // Measured on one B200 (us per op back to back, 40 qubits, complex128, top k =
 // n, target at a high physical bit; before: a launch each for partition,
 // evaluation of every child into 56 bytes of staging per entry, a selection of
 // three histogram passes with grid barriers, and compaction):
-//   n              64   508  16384  65536  300000   2^20   2^22
-//   1-qubit gate   16    16     35     42      65     86    194
-//   before         41    45     63     66      80    108    224
-//   2-qubit gate   26    36     53     66     101    140    308
-//   before         57    62    104    120     135    184    447
-//   rejected step  15    14     34     42      63     75    148
-//   before         41    43     59     62      76     93    201
+//   n              64   508  16384  65536  300000  600000   2^20   2^22
+//   1-qubit gate   14    17     31     35      48      60     89    198
+//   before         38    43     60     64      69      75     91    221
+//   2-qubit gate   30    39     54     58      87     121    147    350
+//   before         55    62     99    113     124     141    171    429
+//   rejected step  12    15     37     38      63      76     75    153
+//   before         41    43     59     69      75      79     95    198
+// (Between 620,000 and 2^20 entries a 1-qubit gate is 3 to 5 per cent slower than
+// before, 9 on the lowest bit: its evaluation then has one tile for every second
+// block.)
 #pragma once
 
 #include <math.h>
@@ -1360,7 +1366,7 @@ __device__ __forceinline__ bool staged_eval(const OpArgs& a, OpSh& sh, const OpC
     for (int u = lane; u < und && u < kQueue; u += 32) undecided(sbase, u, sQueue[w][u]);
     s0.fold();
     s1.fold();
-    if (++folded == 512) {  // the 64-bit integers hold 2^11 tiles of terms below 1
+    if (++folded == 512) {  // the 64-bit integers hold 2^10 tiles of terms below 1 (32 a thread at most)
       limb_add(cn + C_LIMB, s0.get());
       limb_add(cn + C_LIMB + 4, s1.get());
       s0.clear();

@@ -76,12 +76,13 @@ typedef struct bass_state {
 #define BASS_TRACE_WORDS 7 /* u64 per trace event, see bass_ctrl.trace */
 /* Kernel slots of the profiler: 0..29 are the op and tile kernels (kind * 5 +
    pass, kind: 0 gate1, 1 rot1, 2 gate2, 3 perm, 4 plain, 5 rdm; pass: 0 the
-   staged evaluation (rdm: the low-bit pass), 1 its settling, 2 the chip op, 3
-   write, 4 moments), then 30 tile boundaries and sample, 31 workspace clear,
+   staged evaluation (rdm: the low-bit pass), 1 its settling, 2 an op's first
+   launch (a chip op's only one), 3 write, 4 moments), then 30 tile boundaries
+   and sample,
    35 reductions (norm, PR, dot products, the traced rotation commit),
    36 fingerprint, 37 phase2q, 38 phase1q, 39 rdm_final, 40 radix sort,
    41 merge runs, 42 small bookkeeping kernels (dense statevectors among
-   them).  Slots 32-34 and 43-47 are unused and keep the numbering stable. */
+   them).  Slots 31-34 and 43-47 are unused and keep the numbering stable. */
 #define BASS_PROF_SLOTS 48
 
 typedef struct bass_ctrl {
@@ -132,8 +133,15 @@ size_t bass_state_bytes(void);
 size_t bass_ctrl_bytes(void);
 /* workspace for ops whose inputs hold at most max_in entries and whose
    outputs at most max_out entries (before truncation); it is sized for
-   max(4 * max_in, max_out) entries, since the evaluation pass of a 2-qubit
-   gate keeps four 8-byte |a|^2 slots per input entry */
+   max(4 * max_in, max_out) entries, since the staged route of a 2-qubit gate
+   keeps up to four children per input entry.
+   The ws_bytes given to an op also bounds its state's entries (a state of more
+   is refused on the device with BASS_ERR_WORKSPACE), and with that chooses its
+   launches: a state that fits the GPU's shared memory takes one launch if the
+   bound says so, otherwise three more that return at once.  A caller that knows
+   a smaller bound n for a state passes bass_workspace_bytes(ceil(s * n / 4),
+   s * n, num_qubits) of the same buffer, s = 1 for truncations, 2 for 1-qubit
+   ops, 4 for 2-qubit ops. */
 size_t bass_workspace_bytes(int64_t max_in, int64_t max_out, int num_qubits);
 
 /* ---- state management ----------------------------------------------------- */
@@ -266,7 +274,7 @@ int bass_sparse_dot(const bass_state* st, const double* psi, int nq, double* out
    that owns all device memory, a plugin or embedding that may only pass the
    buffers it was given, code that may not call cudaMalloc at that point).  No counterpart in
    the reference.  The scratch is a static array inside the library (about
-   4.8 MB, held on every GPU that loads the library until exit); the state may
+   3.7 MB, held on every GPU that loads the library until exit); the state may
    hold at most 2^20 entries (max_entries is the caller's bound on st->nnz;
    larger values return BASS_ERR_WORKSPACE).  A state that does not fit the
    scratch although max_entries said it would (more than 516 merge tiles,
@@ -332,8 +340,8 @@ typedef struct bass_seg_op {
   int32_t pad;
 } bass_seg_op;
 size_t bass_batch_ws_bytes(int max_ops);
-/* The most states one segmented call takes on the current device (a call's
-   selection keeps one block group per state resident; no counterpart in the
+/* The most states one segmented call takes on the current device (an op's grid
+   barriers keep one block group per state resident; no counterpart in the
    reference, which has no batched path).  0 if no device. */
 int bass_batch_max_segments(void);
 /* bass_gate_1q on every segment (sparse_state.py:15-67 + truncation) */
