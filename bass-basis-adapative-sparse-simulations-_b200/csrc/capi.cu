@@ -296,6 +296,7 @@ int bass_gate_2q(const bass_state* in, bass_state* tmp, bass_state* out, const d
   // pass 1: bring q2 to the lowest physical bit (a pure reorder)
   OpArgs a{};
   a.in = in; a.out = tmp; a.ctrl = ctrl; a.ws = v; a.q = q2; a.gb = 0; a.c64 = state_c64(in);
+  a.entries = v.max_n / 4;
   bass_trunc none{};
   none.k_cond = -1;
   cudaError_t e = run_merge_op(K_PERM, a, none, 0, 0, s);
@@ -319,6 +320,7 @@ int bass_rotate_2q(const bass_state* in, bass_state* tmp, bass_state* out, const
   // pass 1: bring q2 to the lowest physical bit (a pure reorder)
   OpArgs a{};
   a.in = in; a.out = tmp; a.ctrl = ctrl; a.ws = v; a.q = q2; a.gb = 0; a.c64 = state_c64(in);
+  a.entries = v.max_n / 4;
   bass_trunc none{};
   none.k_cond = -1;
   cudaError_t e = run_merge_op(K_PERM, a, none, 0, 0, s);

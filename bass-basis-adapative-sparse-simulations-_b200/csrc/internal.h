@@ -37,6 +37,7 @@ struct OpArgs {
   int commit;     // rotation step: the op also commits (swaps in an accepted candidate)
   int j;          // rotation step: the rotated qubit
   long long k_cond, k_keep;
+  long long entries;  // bound of the state's entries, where it is below what the workspace holds (else 0)
   bass_trunc tr;  // gamma / renormalisation rules
   int c64;        // the input state stores complex64 amplitudes (selects the kernels)
   int rdm_low;    // K_RDM: the qubits at physical bits below kRdmLowBits are left to k_rdm_low

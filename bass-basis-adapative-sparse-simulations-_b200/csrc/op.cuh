@@ -2110,8 +2110,9 @@ static cudaError_t launch_op(OpArgs a, cudaStream_t s) {
   OpGrids g{};
   cudaError_t e = op_grids<KIND, C64>(&g);
   if (e != cudaSuccess) return e;
-  // the workspace bounds the entries (the kernels refuse more)
-  const long long bound = a.ws.max_n / slots_per_entry(KIND);
+  // the workspace bounds the entries (the kernels refuse more); the reorder of a
+  // 2-qubit gate is bounded by the gate after it, which holds a quarter
+  const long long bound = a.entries ? a.entries : a.ws.max_n / slots_per_entry(KIND);
   const bool larger = bound > (long long)g.first * kChipStep<2>;
   a.staged = larger && (!kChip4<KIND> || bound > (long long)g.first4 * kChipStep<4>);
   const long long want = bound <= kChipStep<2> ? 1 : (bound + kChipMin - 1) / kChipMin;
