@@ -78,7 +78,7 @@ const Device& device() {
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct Layout {
-  size_t counters, hist1, hist2, sel, status, fp, red, part, partials, cand_bits, cand_key, tmp_keys,
+  size_t counters, hist1, hist2, hist3, sel, status, fp, red, part, partials, cand_bits, cand_key, tmp_keys,
       tmp_amps, stage_keys, kmask, sort_hist, total;
   long long max_tiles, sort_tiles;
 };
@@ -95,6 +95,7 @@ static Layout layout_for(long long max_n) {
   L.status = o; o += align256((size_t)L.max_tiles * 8);
   L.fp = o; o += align256(8 * 8);
   L.red = o; o += align256(1024 * sizeof(i128));
+  L.hist3 = o; o += align256(kHistBins * 4);
   L.part = o; o += align256((size_t)kMaxSets * (L.max_tiles + 1) * 6 * 8);
   const long long np = (long long)kMaxSets * L.max_tiles > 1024 ? (long long)kMaxSets * L.max_tiles : 1024;
   L.partials = o; o += align256((size_t)np * sizeof(Partial));
@@ -127,6 +128,7 @@ bool carve(void* ws, size_t ws_bytes, WsView* v) {
   v->counters = reinterpret_cast<unsigned int*>(b + L.counters);
   v->hist1 = reinterpret_cast<unsigned int*>(b + L.hist1);
   v->hist2 = reinterpret_cast<unsigned int*>(b + L.hist2);
+  v->hist3 = reinterpret_cast<unsigned int*>(b + L.hist3);
   v->sel = reinterpret_cast<SelState*>(b + L.sel);
   v->status = reinterpret_cast<unsigned long long*>(b + L.status);
   v->fp = reinterpret_cast<unsigned long long*>(b + L.fp);

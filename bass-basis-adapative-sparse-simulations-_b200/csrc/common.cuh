@@ -597,6 +597,7 @@ struct WsView {
   unsigned long long* status;    // max_tiles
   unsigned int* hist1;           // kHistBins bins
   unsigned int* hist2;           // kHistBins bins
+  unsigned int* hist3;           // kHistBins bins (a staged op's sample)
   Partial* partials;             // kMaxSets x max_tiles
   // the staged route's children, per region of a tile (op.cuh), and scratch of others
   unsigned long long* cand_bits; // |a|^2 patterns of the undecided children

@@ -74,8 +74,10 @@ constexpr int kRegions = kThreads / 32;          // regions of a tile
 // A truncation takes one per SM: staged it is slower there (65,536 entries: 51 us
 // instead of 37), and at 2^22 no difference shows.
 constexpr int kFirstBlocks = 64;
-// |a|^2 bins of the sample: 128 per power of two over [2^-64, 1)
+// |a|^2 bins of the sample: 128 per power of two over [2^-64, 1); what lies
+// beyond (in the two outer bins) is also counted four bins to a power of two
 constexpr int kSampleBase = (1023 - 64) << 7;
+constexpr int kFarShift = 50;
 
 // 8-byte words of the workspace counters, zeroed at the start of the op
 enum OpCounter { C_TILE = 0, C_LIST = 1, C_OUT = 2, C_DEF = 3, C_STAGED = 4, C_TILE2 = 5, C_LIMB = 8 };
@@ -1047,7 +1049,10 @@ __device__ __forceinline__ void sample_entry(const OpArgs& a, const OpCtx& X, lo
   const double* amps = reinterpret_cast<const double*>(X.S.amps);
   auto at = [&](long long k) { return amp_get(amps, k, C64, X.r0, X.r1); };
   auto put = [&](double2 c) {
-    atomicAdd(hist + sample_bin((unsigned long long)__double_as_longlong(prob(c)) & 0x7FFFFFFFFFFFFFFFULL), 1u);
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(prob(c)) & 0x7FFFFFFFFFFFFFFFULL;
+    const unsigned b = sample_bin(bits);
+    atomicAdd(hist + b, 1u);
+    if (b == 0 || b == kHistBins - 1) atomicAdd(a.ws.hist3 + (bits >> kFarShift), 1u);
   };
   if (KIND == K_IDENT) {
     if ((threadIdx.x & 7) == 0) put(at(i));
@@ -1124,6 +1129,7 @@ __device__ __forceinline__ void staged_zero(const OpArgs& a, const Grp& g, long 
   for (long long i = gtid; i < kHistBins / 4; i += gthreads) {
     reinterpret_cast<uint4*>(a.ws.hist1)[i] = make_uint4(0, 0, 0, 0);
     reinterpret_cast<uint4*>(a.ws.hist2)[i] = make_uint4(0, 0, 0, 0);
+    reinterpret_cast<uint4*>(a.ws.hist3)[i] = make_uint4(0, 0, 0, 0);
   }
   for (long long i = gtid; i < ntiles; i += gthreads) a.ws.status[i] = 0ULL;
   if (gtid < kOpCounters) reinterpret_cast<unsigned long long*>(a.ws.counters)[gtid] = 0ULL;
@@ -1155,6 +1161,30 @@ __device__ __forceinline__ void staged_prep(const OpArgs& a, const Grp& g, const
   }
 }
 
+// Block-wide: the edges of the sample's bin that holds the r-th child (s, x: the
+// sample's top_scan).  One of the two outer bins is replaced by the quarter of a
+// power of two in it: as a whole it would leave every child of a state with all
+// |a|^2 below 2^-64 undecided (us per 1-qubit gate and truncation of 2^20 entries:
+// 678 and 336 instead of 113 and 83; of 2^22 2164 and 1184 instead of 217 and 146).
+__device__ __forceinline__ void sample_range(const OpArgs& a, FindSh& F, unsigned long long s, unsigned long long x,
+                                             long long r, unsigned long long* lo, unsigned long long* hi) {
+  top_locate<true, kHistBins>(a.ws.hist1, F, s, x, r);
+  const int bin = F.bin;
+  const long long above = F.above;
+  const bool held = above + F.cnt >= r;  // (otherwise fewer children than r)
+  __syncthreads();
+  *lo = held ? sample_edge(bin) : 0ULL;
+  *hi = sample_edge(bin + 1);
+  if (!held || (bin != 0 && bin != kHistBins - 1)) return;
+  // (the highest bin's children come before the lowest one's there)
+  const long long skip = bin == 0 ? (long long)__ldcg(a.ws.hist1 + kHistBins - 1) : 0;
+  find_top<true, kHistBins>(a.ws.hist3, F, skip + r - above);
+  const unsigned long long l = (unsigned long long)F.bin << kFarShift, h = (unsigned long long)(F.bin + 1) << kFarShift;
+  __syncthreads();
+  if (l > *lo) *lo = l;
+  if (h < *hi) *hi = h;
+}
+
 // Block-wide: the bracket, from the sample's histogram (every thread gets it).
 __device__ __forceinline__ Bracket staged_bracket(const OpArgs& a, const Grp& g, const OpCtx& X, FindSh& F) {
   Bracket B{0ULL, 0ULL, 0, 0};  // nothing is dropped: every child certain
@@ -1167,14 +1197,9 @@ __device__ __forceinline__ Bracket staged_bracket(const OpArgs& a, const Grp& g,
   const long long margin = S < n ? (long long)(4.0f * sqrtf((float)S)) : 0;  // four deviations of a rank
   const long long rh = r - margin, rl = r + margin + (S < n ? 1 : 0);
   B.hi = ~0ULL;
-  if (rh >= 1) {
-    top_locate<true, kHistBins>(a.ws.hist1, F, s, x, rh);
-    B.hi = sample_edge(F.bin + 1);
-    __syncthreads();
-  }
-  top_locate<true, kHistBins>(a.ws.hist1, F, s, x, rl);
-  B.lo = F.above + F.cnt >= rl ? sample_edge(F.bin) : 0ULL;
-  __syncthreads();
+  unsigned long long unused;
+  if (rh >= 1) sample_range(a, F, s, x, rh, &unused, &B.hi);
+  sample_range(a, F, s, x, rl, &B.lo, &unused);
   B.shift = digit_shift<kHistBins>(B.lo, B.hi - 1);
   return B;
 }
